@@ -5,10 +5,12 @@
 //   hi.hi + hi.lo + lo.hi recover ~16 (bf16) / ~21 (tf32) significant bits.
 //   D (M x N): fp32, row-major, written with edge masking.
 //
-// Pipeline (persistent: one CTA per SM walks 128 x BN output tiles; BN = 256, 128 or 64; 10 warps):
-//   warp 0      : TMA producer -- cp.async.bulk.tensor.2d into a STAGES-deep ring of 128B-swizzled
-//                 tiles, completion tracked by mbarrier transaction counts;
-//   warp 1      : allocates 2 x BN TMEM columns (two accumulator buffers); one elected thread issues
+// Pipeline (persistent: one CTA per SM walks output tiles of up to 128 x 256; 12 warps):
+//   warps 0, 10, 11 : TMA producers of the P tiles, the Q hi and the Q lo tiles (P = A, Q = B or the other
+//                 way round) -- cp.async.bulk.tensor.2d into a ring of 128B-swizzled tiles, completion
+//                 tracked by mbarrier transaction counts.  One thread issues a copy about every 100 ns,
+//                 which bounds narrow tiles, so the copies of a k-block are shared out;
+//   warp 1      : allocates 512 TMEM columns (two accumulator buffers); one elected thread issues
 //                 tcgen05.mma (kind::f16 for bf16, kind::tf32) from shared-memory descriptors,
 //                 accumulating in TMEM, and frees each ring slot with tcgen05.commit -> mbarrier;
 //   warps 2..9  : epilogue -- tcgen05.ld 32x32b from TMEM (warp w reads lanes 32*(w%4)..+31, half of
@@ -37,7 +39,7 @@ namespace tdscha {
 namespace tc {
 
 constexpr int BM = 128;
-constexpr int NUM_THREADS = 320;   // producer, MMA, 8 epilogue warps
+constexpr int NUM_THREADS = 384;   // P producer, MMA, 8 epilogue warps, 2 Q producers
 constexpr unsigned long long DEFAULT_WAIT_BUDGET_NS = 4000000000ull;   // 4 s per pipeline wait
 constexpr unsigned long long DRAIN_BUDGET_NS = 4000000000ull;          // 4 s per wait of the abort path
 
@@ -72,19 +74,37 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: true when the phase completed, false on timeout or when another role aborted.
+// Bounded wait of a whole warp: true when the phase completed, false (for every lane alike) on timeout
+// or when another role aborted.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                           unsigned long long budget_ns) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
     unsigned long long t0 = 0;
     for (uint32_t it = 0;; ++it) {
-        if (mbar_try(bar, parity)) return true;
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
         if ((it & 255u) == 255u) {
-            if (*abort_flag) return false;
-            unsigned long long t = globaltimer();
+            bool stop = *abort_flag != 0;
+            const unsigned long long t = globaltimer();
             if (t0 == 0) t0 = t;
-            else if (t - t0 > budget_ns) return false;
+            else stop = stop || t - t0 > budget_ns;
+            if (__any_sync(0xffffffffu, stop)) return false;
         }
     }
+}
+// The same for one thread (the abort path's drain).
+__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, unsigned long long budget_ns) {
+    const unsigned long long t0 = globaltimer();
+    while (!mbar_try(bar, parity))
+        if (globaltimer() - t0 > budget_ns) return false;
+    return true;
+}
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(e));
+    return e;
 }
 
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
@@ -116,20 +136,15 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-// Shared-memory matrix descriptor of a K-major tile stored as rows of 128 bytes with the 128-byte
-// swizzle (what TMA writes with CU_TENSOR_MAP_SWIZZLE_128B): start address >> 4 in bits 0-13,
-// leading byte offset (unused for swizzled K-major, 16 B) in bits 16-29, stride byte offset = 1024
-// (one 8-row swizzle atom) in bits 32-45, descriptor version 1 in bits 46-47, swizzle mode 2
-// (128B) in bits 61-63.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)(16u >> 4) << 16;
-    d |= (uint64_t)(1024u >> 4) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= (uint64_t)2u << 61;
-    return d;
-}
+// Shared-memory matrix descriptor of a K-major tile stored as rows of KBYTES (128 or 64) bytes with the
+// swizzle of that width (what TMA writes with CU_TENSOR_MAP_SWIZZLE_128B / _64B): start address >> 4 in
+// bits 0-13, leading byte offset (unused for swizzled K-major, 16 B) in bits 16-29, stride byte offset
+// (one 8-row swizzle atom) in bits 32-45, descriptor version 1 in bits 46-47, swizzle mode (2: 128B,
+// 4: 64B) in bits 61-63.  The high word is the same for every tile, and a step along K or to another
+// tile only adds (bytes >> 4) to the low word (addresses stay below 256 KB).
+template <int KBYTES>
+constexpr uint32_t DESC_HI = ((8u * KBYTES) >> 4) | (1u << 14) | ((KBYTES == 128 ? 2u : 4u) << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
 
 // Instruction descriptor for kind::f16 / kind::tf32 with fp32 accumulation, both operands K-major:
 // D format (bits 4-5) = 1 (f32); A/B format (bits 7-9, 10-12) = 1 (bf16) or 2 (tf32);
@@ -139,23 +154,29 @@ __host__ __device__ constexpr uint32_t make_idesc(bool tf32, int m, int n) {
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-template <bool TF32>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+// issued by the lane whose `leader` is set; the others pass through (no divergent branch, so the
+// descriptors stay in uniform registers)
+template <bool TF32, int KBYTES>
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t adesc, uint32_t bdesc, uint32_t idesc, uint32_t accum, uint32_t leader) {
+    const uint64_t ad = ((uint64_t)DESC_HI<KBYTES> << 32) | adesc, bd = ((uint64_t)DESC_HI<KBYTES> << 32) | bdesc;
     if constexpr (TF32) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(ad), "l"(bd), "r"(idesc), "r"(accum), "r"(leader));
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(ad), "l"(bd), "r"(idesc), "r"(accum), "r"(leader));
     }
 }
 
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(bar), "r"(leader) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -168,17 +189,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Sub-problems of one launch (a single contraction is one group): tile0 = tiles of the groups before.
+// Sub-problems of one launch (a single contraction is one group).  Each 128-row tile of the P operand
+// meets tiles of `tn` rows of the Q operand: P = A, Q = B, or the other way round (swapped).
+// tile0 = tiles of the groups before.
 constexpr int MAX_GROUPS = 64;
 struct DevGroup {
-    int M, N, K, a_row, a_k, b_row, b_k, tile0, num_m, num_n;
+    int np, nq, K, p_row, p_k, q_row, q_k, tile0, num_p, num_q, tn;
     long long d_off;
 };
 struct GroupTable {
     int n, total_tiles;
+    int p_rows;                // P rows of a tile: 128, or 64 (half the P fetch of an MMA, and more tiles)
+    int p_box, q_box;          // rows of one TMA box of each operand
+    int stages, stage_bytes;   // copy ring
+    int q_off;                 // bytes of the stage in front of the Q tiles (hi, then lo)
+    int q_bytes;               // bytes of one Q tile's slot
     DevGroup g[MAX_GROUPS];
 };
 
@@ -188,69 +216,83 @@ __device__ __forceinline__ const DevGroup &group_of(const GroupTable &gt, int t)
     return gt.g[g];
 }
 
-// Tile order of the persistent schedule: groups of `gm` M-tiles, N-tiles of a group in turn, M
-// fastest inside a group.  The ~148 tiles in flight then form a gm x (148/gm) block that shares its
-// A rows and B rows through L2, instead of one N column of tiles streaming all of A from HBM.
-__device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int gm, int &m_blk, int &n_blk) {
-    const int per_group = gm * num_n;
+// Tile order of the persistent schedule: groups of `gp` P-tiles, Q-tiles of a group in turn, P
+// fastest inside a group.  The ~148 tiles in flight then form a gp x (148/gp) block that shares its
+// P rows and Q rows through L2, instead of one Q column of tiles streaming all of P from HBM.
+// Swapped launches keep a P tile's few Q tiles next to each other (gp = 1).
+__device__ __forceinline__ void tile_coords(int t, int num_p, int num_q, int gp, int &p_blk, int &q_blk) {
+    const int per_group = gp * num_q;
     const int g = t / per_group, rem = t % per_group;
-    const int m_first = g * gm;
-    const int rows = min(gm, num_m - m_first);
-    n_blk = rem / rows;
-    m_blk = m_first + rem % rows;
+    const int p_first = g * gp;
+    const int rows = min(gp, num_p - p_first);
+    q_blk = rem / rows;
+    p_blk = p_first + rem % rows;
 }
 
-template <int BN, int STAGES, bool TF32, int NPROD>
-struct Cfg {
-    static constexpr int A_BYTES = BM * 128;                 // one 128 x (128 B) tile
-    static constexpr int B_BYTES = BN * 128;
-    static constexpr int NOPS = (NPROD == 3) ? 2 : 1;        // hi (+ lo)
-    static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-    static constexpr int K_ELEMS = TF32 ? 32 : 64;            // K per stage (128 B of K)
-    static constexpr int UMMA_K = TF32 ? 8 : 16;              // K per instruction (32 B)
-    static constexpr uint32_t TMEM_COLS = 2 * BN;             // two accumulator buffers
-    static constexpr int EPI_WARPS = 8;                       // 2 warps per TMEM lane quadrant
-    static constexpr int EPI_COLS = BN / 2;                   // columns owned by one epilogue thread
-    static constexpr int EPI_BUF_FLOATS = 32 * 32;            // one epilogue warp's 32 x 32 staging block
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ +
-                                      EPI_WARPS * EPI_BUF_FLOATS * 4 /*epilogue staging*/;
-    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of the contraction kernel");
+constexpr int MAX_STAGES = 12;
+constexpr int EPI_WARPS = 8;                       // 2 warps per TMEM lane quadrant
+constexpr int EPI_BUF_FLOATS = 32 * 32;            // one epilogue warp's 32 x 32 staging block
+constexpr int SMEM_MAX = 227 * 1024;
+constexpr int SMEM_FIXED = 1024 /*align*/ + 512 /*barriers*/;
+constexpr int EPI_STAGING = EPI_WARPS * EPI_BUF_FLOATS * 4;
+constexpr uint32_t TMEM_COLS = 512;                // two accumulator buffers of up to 256 columns
+
+template <bool TF32, int KBYTES>
+struct KBlock {
+    static constexpr int ELEMS = KBYTES / (TF32 ? 4 : 2);   // K per stage
+    static constexpr int UMMA_K = TF32 ? 8 : 16;   // K per instruction (32 bytes)
 };
 
-// Persistent: CTA c processes tiles c, c + gridDim.x, ... (m fastest).  Each tile's K loop is split
-// into chunks of `drain` k-blocks; a chunk accumulates from zero in one of two TMEM buffers (the MMA
-// warp moves on to the other buffer) and the epilogue warps add it into round-to-nearest fp32
-// registers, which bounds the error of the tensor core's own fp32 accumulation to `drain` k-blocks.
-template <int BN, int STAGES, bool TF32, int NPROD>
+// Persistent: CTA c processes tiles c, c + gridDim.x, ...  Each tile's K loop is split into chunks
+// of `drain` k-blocks; a chunk accumulates from zero in one of two TMEM buffers (the MMA warp moves on
+// to the other buffer) and the epilogue warps add it into round-to-nearest fp32 registers, which
+// bounds the error of the tensor core's own fp32 accumulation to `drain` k-blocks.
+//
+// What bounds it: large tiles run at the tensor pipe (power-capped); narrow tiles (few output columns,
+// long K) run at the cost of one k-block through the ring, so the MMA warp stays converged (elected
+// issue, uniform descriptors whose low word only gets constants added) and the tile width is whatever
+// the sub-problem needs, in steps of 16 columns, so that no copy, shared memory or MMA goes to padding.
+//   MAXC: columns a tile may have (register accumulators of an epilogue thread = MAXC / 2);
+//   KBYTES: bytes of K of a ring stage.  128, or 64 where stages of 128 would leave the ring two deep
+//         (tiles wider than 192 columns in the split modes): half the shared memory then waits for copies
+//         while the other half computes; four or five half stages keep three quarters of it in flight.
+//         240 rows x 9998 x 512, tf32x3 (Z of five vectors on 3x3x3): 664 -> 596 us.
+//   SWAP: P = B, so that a problem with few rows of A (one chain: 96 or 192 rows) puts them on the
+//         MMA's N side, which steps by 16, instead of padding them to 128-row tiles.
+// The three split products of a k-step are issued hi.hi, A_hi.B_lo, A_lo.B_hi in both orientations and
+// for every width, so each output is the same sum in the same order whatever tile computes it.
+template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
-               const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo,
-               const __grid_constant__ GroupTable gt, int drain, int group_m, float *__restrict__ D, long long ldd, unsigned *err,
+tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant__ CUtensorMap tmP_lo,
+               const __grid_constant__ CUtensorMap tmQ_hi, const __grid_constant__ CUtensorMap tmQ_lo,
+               const __grid_constant__ GroupTable gt, int drain, int group_p, float *__restrict__ D, long long ldd, unsigned *err,
                unsigned *tile_sync, unsigned sync_ns, int accumulate, unsigned long long wait_ns, int stall) {
-    using C = Cfg<BN, STAGES, TF32, NPROD>;
+    using KB = KBlock<TF32, KBYTES>;
+    constexpr int EPI_COLS = MAXC / 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * C::STAGE_BYTES);
-    // bars[0..S) full, [S..2S) empty, [2S, 2S+2) accumulator full, [2S+2, 2S+4) accumulator empty
-    uint64_t *acc_full = bars + 2 * STAGES;
-    uint64_t *acc_empty = bars + 2 * STAGES + 2;
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * STAGES + 4);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 5);
-    uint64_t *done_bar = bars + 2 * STAGES + 6;   // abort path: completion of every MMA issued
-    float *epi_buf = reinterpret_cast<float *>(smem + STAGES * C::STAGE_BYTES + 256);   // epilogue staging blocks
+    const int S = gt.stages, stage_bytes = gt.stage_bytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S * stage_bytes);
+    // bars[0..MS) full, [MS..2MS) empty, then 2 accumulator full, 2 accumulator empty
+    uint64_t *acc_full = bars + 2 * MAX_STAGES;
+    uint64_t *acc_empty = bars + 2 * MAX_STAGES + 2;
+    uint64_t *done_bar = bars + 2 * MAX_STAGES + 4;   // abort path: completion of every MMA issued
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * MAX_STAGES + 5);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * MAX_STAGES + 6);
+    float *epi_buf = reinterpret_cast<float *>(smem + S * stage_bytes + 512);   // epilogue staging blocks
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
     const int num_tiles = gt.total_tiles;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&bars[s]), 1);
-            mbar_init(smem_u32(&bars[STAGES + s]), 1);
+        for (int s = 0; s < S; ++s) {
+            mbar_init(smem_u32(&bars[s]), NPROD == 3 ? 3 : 2);   // one arrival per producer warp
+            mbar_init(smem_u32(&bars[MAX_STAGES + s]), 1);
         }
         for (int x = 0; x < 2; ++x) {
             mbar_init(smem_u32(&acc_full[x]), 1);
-            mbar_init(smem_u32(&acc_empty[x]), C::EPI_WARPS);
+            mbar_init(smem_u32(&acc_empty[x]), EPI_WARPS);
         }
         mbar_init(smem_u32(done_bar), 1);
         *abort_flag = 0;
@@ -258,115 +300,147 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(tmem_slot)), "r"(C::TMEM_COLS) : "memory");
+                     ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t bar0 = smem_u32(bars), smem0 = smem_u32(smem);
 
-    long long issued = 0;   // k-blocks handed to TMA by the producer (for the drain on abort)
-    if (warp == 0 && lane == 0 && !stall) {
-        // ---------------- TMA producer ----------------
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA_hi)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB_hi)) : "memory");
-        long long g = 0;
+    int issued = 0;      // k-blocks this producer handed to TMA (for the drain on abort)
+    if ((warp == 0 || warp == 10 || (warp == 11 && NPROD == 3)) && !stall) {
+        // ---------------- TMA producers: P (hi and lo), Q hi, Q lo ----------------
+        const uint32_t leader = elect_one();
+        const CUtensorMap *map = warp == 0 ? &tmP_hi : (warp == 10 ? &tmQ_hi : &tmQ_lo);
+        if (leader) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+        const uint32_t dst0 = smem0 + (warp == 0 ? 0 : gt.q_off + (warp == 10 ? 0 : gt.q_bytes));
+        int s = 0;
+        uint32_t ph = 1;
         unsigned target = 0;   // tile starts of all CTAs up to and including this round
-        for (int t = blockIdx.x, round = 0; t < num_tiles && !*abort_flag; t += gridDim.x, ++round) {
-            target += (unsigned)min((int)gridDim.x, num_tiles - round * (int)gridDim.x);
-            if (tile_sync) tile_start_sync(tile_sync, target, round > 0 ? sync_ns : 0ull);
-            const DevGroup &G = group_of(gt, t);
-            int mb, nbk;
-            tile_coords(t - G.tile0, G.num_m, G.num_n, group_m, mb, nbk);
-            const int m0 = G.a_row + mb * BM, n0 = G.b_row + nbk * BN;
-            const int num_kb = G.K / C::K_ELEMS;
-            for (int kb = 0; kb < num_kb; ++kb, ++g) {
-                const int s = (int)(g % STAGES);
-                const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-                if (!mbar_wait(smem_u32(&bars[STAGES + s]), ph ^ 1u, abort_flag, wait_ns)) { *abort_flag = 1; break; }
-                uint8_t *st = smem + s * C::STAGE_BYTES;
-                const uint32_t full = smem_u32(&bars[s]);
-                mbar_expect_tx(full, C::STAGE_BYTES);
-                const int kc = kb * C::K_ELEMS;
-                tma_load_2d(smem_u32(st), &tmA_hi, G.a_k + kc, m0, full);
-                tma_load_2d(smem_u32(st + C::NOPS * C::A_BYTES), &tmB_hi, G.b_k + kc, n0, full);
-                if constexpr (NPROD == 3) {
-                    tma_load_2d(smem_u32(st + C::A_BYTES), &tmA_lo, G.a_k + kc, m0, full);
-                    tma_load_2d(smem_u32(st + C::NOPS * C::A_BYTES + C::B_BYTES), &tmB_lo, G.b_k + kc, n0, full);
-                }
-                issued = g + 1;
-            }
-        }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer ----------------
-        constexpr uint32_t idesc = make_idesc(TF32, BM, BN);
-        long long g = 0, ch = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-            const int num_kb = group_of(gt, t).K / C::K_ELEMS;
-            const int chunks_per_tile = (num_kb + drain - 1) / drain;
-            for (int c = 0; c < chunks_per_tile && ok; ++c, ++ch) {
-                const int X = (int)(ch & 1);
-                const uint32_t use = (uint32_t)(ch >> 1);
-                if (!mbar_wait(smem_u32(&acc_empty[X]), (use & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t dtm = tmem_base + (uint32_t)(X * BN);
-                const int kb_end = min(num_kb, (c + 1) * drain);
-                for (int kb = c * drain; kb < kb_end; ++kb, ++g) {
-                    const int s = (int)(g % STAGES);
-                    const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-                    if (!mbar_wait(smem_u32(&bars[s]), ph, abort_flag, wait_ns)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    uint8_t *st = smem + s * C::STAGE_BYTES;
-                    const uint32_t a_hi = smem_u32(st);
-                    const uint32_t b_hi = smem_u32(st + C::NOPS * C::A_BYTES);
-#pragma unroll
-                    for (int k = 0; k < C::K_ELEMS / C::UMMA_K; ++k) {
-                        const uint32_t koff = k * 32;   // bytes inside the 128-byte swizzled row
-                        const uint32_t acc = (kb > c * drain || k > 0) ? 1u : 0u;
-                        umma<TF32>(dtm, sw128_desc(a_hi + koff), sw128_desc(b_hi + koff), idesc, acc);
-                        if constexpr (NPROD == 3) {
-                            const uint32_t a_lo = smem_u32(st + C::A_BYTES);
-                            const uint32_t b_lo = smem_u32(st + C::NOPS * C::A_BYTES + C::B_BYTES);
-                            umma<TF32>(dtm, sw128_desc(a_hi + koff), sw128_desc(b_lo + koff), idesc, 1u);
-                            umma<TF32>(dtm, sw128_desc(a_lo + koff), sw128_desc(b_hi + koff), idesc, 1u);
-                        }
+        for (int t = blockIdx.x, round = 0; t < num_tiles && ok; t += gridDim.x, ++round) {
+            target += (unsigned)min((int)gridDim.x, num_tiles - round * (int)gridDim.x);
+            if (tile_sync && warp == 0) {
+                if (leader) tile_start_sync(tile_sync, target, round > 0 ? sync_ns : 0ull);
+                __syncwarp();
+            }
+            const DevGroup &G = group_of(gt, t);
+            int pb, qb;
+            tile_coords(t - G.tile0, G.num_p, G.num_q, group_p, pb, qb);
+            const int num_kb = G.K / KB::ELEMS;
+            int row, kc, nbox, box;
+            if (warp == 0) {
+                row = G.p_row + pb * gt.p_rows;
+                kc = G.p_k;
+                box = gt.p_box;
+                nbox = 1;
+            } else {
+                row = G.q_row + qb * G.tn;
+                kc = G.q_k;
+                box = gt.q_box;
+                nbox = (min(G.tn, G.nq - qb * G.tn) + box - 1) / box;
+            }
+            const uint32_t tx = (uint32_t)((warp == 0 && NPROD == 3 ? 2 : nbox) * box * KBYTES);
+            for (int kb = 0; kb < num_kb; ++kb, kc += KB::ELEMS) {
+                if (!mbar_wait(bar0 + 8 * (MAX_STAGES + s), ph, abort_flag, wait_ns)) { ok = false; break; }
+                if (leader) {
+                    const uint32_t dst = dst0 + s * stage_bytes, full = bar0 + 8 * s;
+                    mbar_expect_tx(full, tx);
+                    tma_load_2d(dst, map, kc, row, full);
+                    if (warp == 0) {
+                        if constexpr (NPROD == 3) tma_load_2d(dst + (gt.q_off >> 1), &tmP_lo, kc, row, full);
+                    } else {
+                        for (int i = 1; i < nbox; ++i) tma_load_2d(dst + i * box * KBYTES, map, kc, row + i * box, full);
                     }
-                    umma_commit(smem_u32(&bars[STAGES + s]));   // slot s free once these MMAs retire
                 }
-                if (!ok) break;
-                umma_commit(smem_u32(&acc_full[X]));             // chunk accumulated in buffer X
+                ++issued;
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
         if (!ok) *abort_flag = 1;
-    } else if (warp >= 2) {
-        // ---------------- epilogue: drain chunks into fp32 registers, store each tile ----------------
-        const int ew = warp - 2;
-        const int q = warp & 3;              // TMEM lane quadrant this warp may access
-        const int half = ew >> 2;            // which half of the BN columns this warp owns
-        long long ch = 0;
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        const uint32_t leader = elect_one();
+        const uint32_t desc0 = desc_lo(smem0), stage_d = (uint32_t)stage_bytes >> 4;
+        const uint32_t d_plo = (uint32_t)gt.q_off >> 5, d_qhi = (uint32_t)gt.q_off >> 4;
+        const uint32_t d_qlo = d_qhi + ((uint32_t)gt.q_bytes >> 4);
+        int s = 0;
+        uint32_t ph = 0, ch = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
             const DevGroup &G = group_of(gt, t);
-            int mb, nbk;
-            tile_coords(t - G.tile0, G.num_m, G.num_n, group_m, mb, nbk);
-            const int m0 = mb * BM, n0 = nbk * BN;
-            const int M = G.M, N = G.N;
-            const int chunks_per_tile = (G.K / C::K_ELEMS + drain - 1) / drain;
-            float acc[C::EPI_COLS];
-#pragma unroll
-            for (int i = 0; i < C::EPI_COLS; ++i) acc[i] = 0.f;
-            for (int c = 0; c < chunks_per_tile; ++c, ++ch) {
-                const int X = (int)(ch & 1);
-                const uint32_t use = (uint32_t)(ch >> 1);
-                if (!mbar_wait(smem_u32(&acc_full[X]), use & 1u, abort_flag, wait_ns)) { ok = false; break; }
+            int pb, qb;
+            tile_coords(t - G.tile0, G.num_p, G.num_q, group_p, pb, qb);
+            const int ncol = (min(G.tn, G.nq - qb * G.tn) + 15) & ~15;
+            const uint32_t idesc = make_idesc(TF32, gt.p_rows, ncol);
+            const int num_kb = G.K / KB::ELEMS;
+            for (int k0 = 0; k0 < num_kb && ok; k0 += drain, ++ch) {
+                const uint32_t X = ch & 1u;
+                if (!mbar_wait(smem_u32(&acc_empty[X]), ((ch >> 1) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(X * BN + half * C::EPI_COLS);
+                const uint32_t dtm = tmem_base + X * 256u;
+                const int kb_end = min(num_kb, k0 + drain);
+                uint32_t acc = 0;
+                for (int kb = k0; kb < kb_end; ++kb) {
+                    if (!mbar_wait(bar0 + 8 * s, ph, abort_flag, wait_ns)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t d = desc0 + (uint32_t)s * stage_d;
 #pragma unroll
-                for (int sub = 0; sub < C::EPI_COLS / 32; ++sub) {
+                    for (int k = 0; k < KB::ELEMS / KB::UMMA_K; ++k) {
+                        const uint32_t ko = k * 2;   // 32 bytes inside the swizzled row, >> 4
+                        umma<TF32, KBYTES>(dtm, d + ko, d + d_qhi + ko, idesc, k > 0 ? 1u : acc, leader);
+                        if constexpr (NPROD == 3) {
+                            if constexpr (!SWAP) {
+                                umma<TF32, KBYTES>(dtm, d + ko, d + d_qlo + ko, idesc, 1u, leader);
+                                umma<TF32, KBYTES>(dtm, d + d_plo + ko, d + d_qhi + ko, idesc, 1u, leader);
+                            } else {
+                                umma<TF32, KBYTES>(dtm, d + d_plo + ko, d + d_qhi + ko, idesc, 1u, leader);
+                                umma<TF32, KBYTES>(dtm, d + ko, d + d_qlo + ko, idesc, 1u, leader);
+                            }
+                        }
+                    }
+                    acc = 1;
+                    umma_commit(bar0 + 8 * (MAX_STAGES + s), leader);   // slot s free once these MMAs retire
+                    if (++s == S) { s = 0; ph ^= 1u; }
+                }
+                if (!ok) break;
+                umma_commit(smem_u32(&acc_full[X]), leader);             // chunk accumulated in buffer X
+            }
+        }
+        if (!ok) *abort_flag = 1;
+    } else if (warp >= 2 && warp < 10) {
+        // ---------------- epilogue: drain chunks into fp32 registers, store each tile ----------------
+        const int ew = warp - 2;
+        const int q = warp & 3;              // TMEM lane quadrant this warp may access
+        const int half = ew >> 2;            // which half of the tile's columns this warp owns
+        uint32_t ch = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+            const DevGroup &G = group_of(gt, t);
+            int pb, qb;
+            tile_coords(t - G.tile0, G.num_p, G.num_q, group_p, pb, qb);
+            const int width = min(G.tn, G.nq - qb * G.tn);          // valid columns of this tile
+            const int hw = ((width + 63) >> 6) << 5;                // columns of a half, a multiple of 32
+            const int c_lo = half * hw;
+            const int nsub = (min(hw, width - c_lo) + 31) >> 5;     // 32-column pieces of this warp
+            const int rq = gt.p_rows >> 2;                          // P rows of a lane quadrant: 32, or 16 (lanes 0..15)
+            const int num_kb = G.K / KB::ELEMS;
+            float acc[EPI_COLS];
+#pragma unroll
+            for (int i = 0; i < EPI_COLS; ++i) acc[i] = 0.f;
+            for (int k0 = 0; k0 < num_kb; k0 += drain, ++ch) {
+                const uint32_t X = ch & 1u;
+                if (!mbar_wait(smem_u32(&acc_full[X]), (ch >> 1) & 1u, abort_flag, wait_ns)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + X * 256u + (uint32_t)c_lo;
+#pragma unroll
+                for (int sub = 0; sub < EPI_COLS / 32; ++sub) {
+                    if (sub >= nsub) break;
                     uint32_t r[32];
                     tmem_ld32(tbase + (uint32_t)(sub * 32), r);
+                    tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 32; ++i) acc[sub * 32 + i] += __uint_as_float(r[i]);
                 }
@@ -375,45 +449,66 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[X])) : "memory");
             }
             if (!ok) break;
-            // Store through this warp's 32 x 32 staging block: each lane writes its row's 32 columns, then
-            // lanes 8i..8i+7 store 128 contiguous bytes of one row each, so one store instruction covers
-            // four full 128-byte lines instead of 16 bytes of 32 rows.  16-byte chunks are XOR-swizzled by
-            // row (chunk j of row r at j ^ (r & 7)), which keeps both phases free of bank conflicts.
-            float *wbuf = epi_buf + ew * C::EPI_BUF_FLOATS;
-            const int cb0 = n0 + half * C::EPI_COLS;
-            const bool vec = ((ldd & 3) == 0) && ((G.d_off & 3) == 0);
-            const int rsub = lane >> 3, chk = lane & 7;
+            if constexpr (SWAP) {
+                // lane = output column (P row), register = output row (Q row): each register is one
+                // coalesced 128-byte store of the warp
+                const int m = pb * gt.p_rows + q * rq + lane;
+                if (lane < rq && m < G.np) {
+                    float *dcol = D + G.d_off + (long long)(qb * G.tn + c_lo) * ldd + m;
 #pragma unroll
-            for (int sub = 0; sub < C::EPI_COLS / 32; ++sub) {
+                    for (int sub = 0; sub < EPI_COLS / 32; ++sub) {
+                        if (sub >= nsub) break;
+                        const int left = width - c_lo - sub * 32;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    *reinterpret_cast<float4 *>(wbuf + lane * 32 + 4 * (j ^ (lane & 7))) =
-                        make_float4(acc[sub * 32 + 4 * j], acc[sub * 32 + 4 * j + 1], acc[sub * 32 + 4 * j + 2],
-                                    acc[sub * 32 + 4 * j + 3]);
-                __syncwarp();
-                const int cb = cb0 + sub * 32 + 4 * chk;
-#pragma unroll 1
-                for (int i0 = 0; i0 < 32; i0 += 4) {
-                    const int i = i0 + rsub;
-                    const float4 v = *reinterpret_cast<const float4 *>(wbuf + i * 32 + 4 * (chk ^ (i & 7)));
-                    const long long grow = (long long)m0 + q * 32 + i;
-                    if (grow >= M) continue;
-                    float *drow = D + G.d_off + grow * ldd;
-                    if (vec && cb + 4 <= N) {
-                        float4 o = v;
-                        if (accumulate) {
-                            const float4 old = *reinterpret_cast<const float4 *>(drow + cb);
-                            o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                        }
-                        *reinterpret_cast<float4 *>(drow + cb) = o;
-                    } else {
-                        const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (cb + e < N) drow[cb + e] = accumulate ? drow[cb + e] + vv[e] : vv[e];
+                        for (int i = 0; i < 32; ++i)
+                            if (i < left) {
+                                float *d = dcol + (long long)(sub * 32 + i) * ldd;
+                                *d = accumulate ? *d + acc[sub * 32 + i] : acc[sub * 32 + i];
+                            }
                     }
                 }
-                __syncwarp();   // the block is rewritten by the next 32 columns
+            } else {
+                // Store through this warp's 32 x 32 staging block: each lane writes its row's 32 columns, then
+                // lanes 8i..8i+7 store 128 contiguous bytes of one row each, so one store instruction covers
+                // four full 128-byte lines instead of 16 bytes of 32 rows.  16-byte chunks are XOR-swizzled by
+                // row (chunk j of row r at j ^ (r & 7)), which keeps both phases free of bank conflicts.
+                const int m0 = pb * gt.p_rows + q * rq, cb0 = qb * G.tn + c_lo, c_end = qb * G.tn + width;
+                float *wbuf = epi_buf + ew * EPI_BUF_FLOATS;
+                const bool vec = ((ldd & 3) == 0) && ((G.d_off & 3) == 0);
+                const int rsub = lane >> 3, chk = lane & 7;
+#pragma unroll
+                for (int sub = 0; sub < EPI_COLS / 32; ++sub) {
+                    if (sub >= nsub) break;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<float4 *>(wbuf + lane * 32 + 4 * (j ^ (lane & 7))) =
+                            make_float4(acc[sub * 32 + 4 * j], acc[sub * 32 + 4 * j + 1], acc[sub * 32 + 4 * j + 2],
+                                        acc[sub * 32 + 4 * j + 3]);
+                    __syncwarp();
+                    const int cb = cb0 + sub * 32 + 4 * chk;
+#pragma unroll 1
+                    for (int i0 = 0; i0 < rq; i0 += 4) {
+                        const int i = i0 + rsub;
+                        const float4 v = *reinterpret_cast<const float4 *>(wbuf + i * 32 + 4 * (chk ^ (i & 7)));
+                        const long long grow = (long long)m0 + i;
+                        if (grow >= G.np) continue;
+                        float *drow = D + G.d_off + grow * ldd;
+                        if (vec && cb + 4 <= c_end) {
+                            float4 o = v;
+                            if (accumulate) {
+                                const float4 old = *reinterpret_cast<const float4 *>(drow + cb);
+                                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+                            }
+                            *reinterpret_cast<float4 *>(drow + cb) = o;
+                        } else {
+                            const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (cb + e < c_end) drow[cb + e] = accumulate ? drow[cb + e] + vv[e] : vv[e];
+                        }
+                    }
+                    __syncwarp();   // the block is rewritten by the next 32 columns
+                }
             }
         }
         if (!ok) *abort_flag = 1;
@@ -424,23 +519,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     __syncthreads();
     if (*abort_flag) {
         if (threadIdx.x == 0) atomicOr(err, ERR_TIMEOUT);
-        volatile int never = 0;
-        if (warp == 0 && lane == 0) {
+        if ((warp == 0 || warp >= 10) && lane == 0) {
             // drain the TMA copies this CTA still has in flight (bounded; copies older than the last
-            // STAGES completed before their slots were handed back)
-            for (long long g = (issued > STAGES ? issued - STAGES : 0); g < issued; ++g)
-                mbar_wait(smem_u32(&bars[g % STAGES]), (uint32_t)(g / STAGES) & 1u, &never, DRAIN_BUDGET_NS);
+            // `stages` completed before their slots were handed back)
+            for (int g = (issued > S ? issued - S : 0); g < issued; ++g)
+                mbar_wait_thread(bar0 + 8 * (g % S), (uint32_t)(g / S) & 1u, DRAIN_BUDGET_NS);
         }
-        if (warp == 1 && lane == 0) {
-            // every MMA this thread issued has retired before the accumulator columns are released
-            umma_commit(smem_u32(done_bar));
-            mbar_wait(smem_u32(done_bar), 0u, &never, DRAIN_BUDGET_NS);
+        if (warp == 1) {
+            // every MMA the elected lane issued has retired before the accumulator columns are released
+            const uint32_t leader = elect_one();
+            umma_commit(smem_u32(done_bar), leader);
+            if (leader) mbar_wait_thread(smem_u32(done_bar), 0u, DRAIN_BUDGET_NS);
+            __syncwarp();
         }
         __syncthreads();
     }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -463,8 +559,8 @@ static EncodeTiledFn get_encode() {
     return fn;
 }
 
-// rows x K operand, leading dimension ld (elements), box = box_rows x (128 bytes of K)
-static int make_map(CUtensorMap *map, const void *base, bool tf32, long long rows, long long K, long long ld, int box_rows) {
+// rows x K operand, leading dimension ld (elements), box = box_rows x (kbytes of K)
+static int make_map(CUtensorMap *map, const void *base, bool tf32, long long rows, long long K, long long ld, int box_rows, int kbytes) {
     EncodeTiledFn enc = get_encode();
     TD_CHECK(enc != nullptr, TDSCHA_ECUDA, "cuTensorMapEncodeTiled entry point unavailable");
     const size_t es = tf32 ? 4 : 2;
@@ -472,11 +568,11 @@ static int make_map(CUtensorMap *map, const void *base, bool tf32, long long row
     TD_CHECK(((ld * es) & 15) == 0, TDSCHA_EINVAL, "operand row stride not a multiple of 16 bytes");
     cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     cuuint64_t gstride[1] = {(cuuint64_t)(ld * es)};
-    cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)(kbytes / es), (cuuint32_t)box_rows};
     cuuint32_t estride[2] = {1, 1};
     CUresult r = enc(map, tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                      const_cast<void *>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     kbytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TD_CHECK(r == CUDA_SUCCESS, TDSCHA_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return 0;
@@ -534,204 +630,311 @@ static unsigned tile_sync_budget_ns() {
     return (unsigned)v;
 }
 
-// One tile configuration of a contraction, ready to launch with a tile-group size.
-struct Prepared {
-    std::function<void(int)> launch;
-    int num_m = 0;
-    int bn = 0;            // tile width (outputs per tile along N)
-    long long tiles = 0;
-};
-
 // Extents of the two operand buffers and the sub-problems of one contraction.
 struct Problem {
     long long a_rows, a_cols, b_rows, b_cols;
     std::vector<GemmGroup> groups;
 };
 
-template <int BN, int STAGES, bool TF32, int NPROD>
-static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, size_t g1, float *D, long long ldd,
-                       cudaStream_t st, unsigned *err, unsigned *counter, int stall, Prepared *out) {
-    using C = Cfg<BN, STAGES, TF32, NPROD>;
-    CUtensorMap a_hi, a_lo, b_hi, b_lo;
-    TD_TRY(make_map(&a_hi, op.A_hi, TF32, pb.a_rows, pb.a_cols, op.lda, BM));
-    TD_TRY(make_map(&b_hi, op.B_hi, TF32, pb.b_rows, pb.b_cols, op.ldb, BN));
-    if (NPROD == 3) {
-        TD_TRY(make_map(&a_lo, op.A_lo, TF32, pb.a_rows, pb.a_cols, op.lda, BM));
-        TD_TRY(make_map(&b_lo, op.B_lo, TF32, pb.b_rows, pb.b_cols, op.ldb, BN));
-    } else {
-        a_lo = a_hi;
-        b_lo = b_hi;
+// A tile shape: orientation and the widest tile along the MMA's N side.
+struct TileShape {
+    bool swap = false;   // the 128-row side of a tile is B (output columns) instead of A (output rows)
+    int cap = 256;       // columns of a tile at most
+    int p_rows = BM;     // P rows of a tile (128 or 64)
+};
+
+// Width of the tiles that cover n columns in pieces of at most cap: equal pieces, a multiple of 16.
+static int tile_width(int n, int cap) { return (int)round_up(ceil_div(n, ceil_div(n, cap)), 16); }
+
+struct TilePlan {
+    long long tiles = 0;
+    int p_box = 128, q_box = 0, q_rows = 0, max_p = 1;
+    double cycles = 0;   // estimated SM cycles of the launch
+};
+
+// Tiles, TMA boxes and estimated time of groups [g0, g1) with one tile shape.  The estimate (SM cycles
+// of a k-block: the largest of its MMA time, its copy time and the ring's latency) only has to order
+// the shapes; measured on this GPU with one tile per SM: an MMA instruction takes half a cycle per
+// column but no less than 68 cycles for its 128 P rows (34 for 64), copies 60 B per cycle and SM.
+static TilePlan plan_tiles(const Problem &pb, size_t g0, size_t g1, TileShape sh, int kelems, int nprod, int drain, int sms) {
+    TilePlan pl;
+    const int nops = nprod == 3 ? 2 : 1;
+    int pmax = 1;
+    for (size_t i = g0; i < g1; ++i) pmax = std::max(pmax, sh.swap ? pb.groups[i].N : pb.groups[i].M);
+    pl.p_box = (int)std::min<long long>(sh.p_rows, round_up(pmax, 8));
+    // one Q box height for every group: the least rows copied, fewer boxes on a tie
+    double best = 1e300;
+    for (int q = 16; q <= 256; q += 16) {
+        double cost = 0;
+        int rows_max = 0;
+        for (size_t i = g0; i < g1 && rows_max <= 256; ++i) {
+            const GemmGroup &G = pb.groups[i];
+            const int nq = sh.swap ? G.M : G.N, np = sh.swap ? G.N : G.M;
+            const int tn = tile_width(nq, sh.cap), boxes = ceil_div(tn, q);
+            rows_max = std::max(rows_max, boxes * q);
+            cost += (double)ceil_div(nq, tn) * ceil_div(np, sh.p_rows) * G.K * (boxes * q + 8.0 * boxes);
+        }
+        if (rows_max > 256) continue;
+        if (cost < best) { best = cost; pl.q_box = q; pl.q_rows = rows_max; }
     }
+    double total = 0, longest = 0;
+    for (size_t i = g0; i < g1; ++i) {
+        const GemmGroup &G = pb.groups[i];
+        const int nq = sh.swap ? G.M : G.N, np = sh.swap ? G.N : G.M;
+        const int tn = tile_width(nq, sh.cap);
+        const int num_p = ceil_div(np, sh.p_rows), num_q = ceil_div(nq, tn), nkb = G.K / kelems;
+        const double mma = 4.0 * nprod * std::max(tn * 0.5, sh.p_rows * 0.53);
+        const double copy = nops * 128.0 * (pl.p_box + ceil_div(tn, pl.q_box) * pl.q_box) / 60.0;
+        const double lat = 400.0 + 150.0 / drain;
+        const double tile = nkb * std::max(mma, std::max(copy, lat)) + 1500.0 + (sh.swap ? 40.0 : 16.0) * tn;
+        pl.tiles += (long long)num_p * num_q;
+        pl.max_p = std::max(pl.max_p, num_p);
+        total += tile * num_p * num_q;
+        longest = std::max(longest, tile);
+    }
+    const double per_sm = total / sms, waves = (double)((pl.tiles + sms - 1) / sms) * (total / pl.tiles);
+    pl.cycles = std::max(longest, 0.5 * (per_sm + std::max(per_sm, waves)));
+    return pl;
+}
+
+// One tile shape of a contraction, ready to launch with a tile-group size.
+struct Prepared {
+    std::function<void(int)> launch;
+    int num_p = 0;
+    TileShape shape;
+    long long tiles = 0;
+};
+
+template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES>
+static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
+                       long long ldd, cudaStream_t st, unsigned *err, unsigned *counter, int stall, int sms, Prepared *out) {
+    CUtensorMap p_hi, p_lo, q_hi, q_lo;
+    const int a_box = SWAP ? pl.q_box : pl.p_box, b_box = SWAP ? pl.p_box : pl.q_box;
+    CUtensorMap *a_maps[2] = {SWAP ? &q_hi : &p_hi, SWAP ? &q_lo : &p_lo}, *b_maps[2] = {SWAP ? &p_hi : &q_hi, SWAP ? &p_lo : &q_lo};
+    TD_TRY(make_map(a_maps[0], op.A_hi, TF32, pb.a_rows, pb.a_cols, op.lda, a_box, KBYTES));
+    TD_TRY(make_map(b_maps[0], op.B_hi, TF32, pb.b_rows, pb.b_cols, op.ldb, b_box, KBYTES));
+    if (NPROD == 3) {
+        TD_TRY(make_map(a_maps[1], op.A_lo, TF32, pb.a_rows, pb.a_cols, op.lda, a_box, KBYTES));
+        TD_TRY(make_map(b_maps[1], op.B_lo, TF32, pb.b_rows, pb.b_cols, op.ldb, b_box, KBYTES));
+    } else {
+        p_lo = p_hi;
+        q_lo = q_hi;
+    }
+    constexpr int NOPS = NPROD == 3 ? 2 : 1;
     GroupTable gt{};
     gt.n = (int)(g1 - g0);
+    gt.p_rows = sh.p_rows;
+    gt.p_box = pl.p_box;
+    gt.q_box = pl.q_box;
+    gt.q_off = NOPS * sh.p_rows * KBYTES;
+    gt.q_bytes = pl.q_rows * KBYTES;
+    gt.stage_bytes = gt.q_off + NOPS * gt.q_bytes;
+    const int staging = SWAP ? 0 : EPI_STAGING;
+    gt.stages = std::min(MAX_STAGES, (SMEM_MAX - SMEM_FIXED - staging) / gt.stage_bytes);
+    TD_CHECK(gt.stages >= 2, TDSCHA_EINVAL, "tc::gemm: tile of %d rows does not fit", pl.q_rows);
+    const int smem = gt.stages * gt.stage_bytes + SMEM_FIXED + staging;
     long long tiles = 0;
-    int max_m = 1;
     for (size_t i = g0; i < g1; ++i) {
-        const GemmGroup &q = pb.groups[i];
+        const GemmGroup &g = pb.groups[i];
         DevGroup &d = gt.g[i - g0];
-        d.M = q.M; d.N = q.N; d.K = q.K;
-        d.a_row = q.a_row; d.a_k = q.a_k; d.b_row = q.b_row; d.b_k = q.b_k;
-        d.d_off = q.d_off;
-        d.num_m = ceil_div(q.M, BM);
-        d.num_n = ceil_div(q.N, BN);
+        d.np = SWAP ? g.N : g.M;
+        d.nq = SWAP ? g.M : g.N;
+        d.K = g.K;
+        d.p_row = SWAP ? g.b_row : g.a_row;
+        d.p_k = SWAP ? g.b_k : g.a_k;
+        d.q_row = SWAP ? g.a_row : g.b_row;
+        d.q_k = SWAP ? g.a_k : g.b_k;
+        d.d_off = g.d_off;
+        d.tn = tile_width(d.nq, sh.cap);
+        d.num_p = ceil_div(d.np, sh.p_rows);
+        d.num_q = ceil_div(d.nq, d.tn);
         d.tile0 = (int)tiles;
-        tiles += (long long)d.num_m * d.num_n;
-        max_m = std::max(max_m, d.num_m);
+        tiles += (long long)d.num_p * d.num_q;
     }
     TD_CHECK(tiles < (1LL << 31), TDSCHA_EINVAL, "tc::gemm: %lld tiles exceed the schedule", tiles);
     gt.total_tiles = (int)tiles;
-    auto kern = tc_gemm_kernel<BN, STAGES, TF32, NPROD>;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-    int dev = 0, sms = 148;
+    auto kern = tc_gemm_kernel<MAXC, TF32, NPROD, SWAP, KBYTES>;
+    static std::atomic<unsigned long long> attr_set{0};   // one bit per device
+    int dev = 0;
     TD_CUDA(cudaGetDevice(&dev));
-    TD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int drain = op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD);
+    if (dev >= 64 || !((attr_set.load() >> dev) & 1ull)) {
+        TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+        if (dev < 64) attr_set.fetch_or(1ull << dev);
+    }
+    const int drain = (op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD)) * (128 / KBYTES);   // in stages
     const dim3 grid((unsigned)std::min<long long>(tiles, sms));
     const unsigned sync_ns = tile_sync_budget_ns();
     const int accumulate = op.accumulate ? 1 : 0;
     const unsigned long long wait_ns = g_wait_budget_ns.load();
-    unsigned *cnt = (sync_ns > 0 && tiles > grid.x) ? counter : nullptr;
-    out->num_m = max_m;
-    out->bn = BN;
+    // Tile starts are aligned only where K is long: the panels of one tile then outgrow L2 and CTAs that
+    // drift apart re-read them.  Below that the wait and its counter's memset only cost: [a|b] of 192
+    // rows x 20000, K <= 2432: 1623 us aligned, 1564 us not; Z (K = 20032) the same either way.
+    int k_max = 0;
+    for (size_t i = g0; i < g1; ++i) k_max = std::max(k_max, pb.groups[i].K);
+    unsigned *cnt = (sync_ns > 0 && tiles > grid.x && k_max >= 32768) ? counter : nullptr;
+    out->num_p = pl.max_p;
+    out->shape = sh;
     out->tiles = tiles;
-    out->launch = [=](int gm) {
+    out->launch = [=](int gp) {
         if (cnt) cudaMemsetAsync(cnt, 0, sizeof(unsigned), st);
-        kern<<<grid, NUM_THREADS, C::SMEM_BYTES, st>>>(a_hi, a_lo, b_hi, b_lo, gt, drain, gm, D, ldd, err, cnt, sync_ns,
-                                                        accumulate, wait_ns, stall);
+        kern<<<grid, NUM_THREADS, smem, st>>>(p_hi, p_lo, q_hi, q_lo, gt, drain, gp, D, ldd, err, cnt, sync_ns, accumulate, wait_ns,
+                                              stall);
     };
     return 0;
 }
 
-// ---- tile-shape and tile-order autotuner -----------------------------------------------------------
-// On the first call for a (format, products, M, N, K) the launcher times every candidate (tile
-// configuration, tile-group size) on the caller's stream and remembers the winner: the candidates run
-// in turn, twice round (every run writes the same D), and each keeps its faster run, so that the clock
-// drift of a power-capped GPU over the trials does not favour the candidates timed first.
-// TDSCHA_AUTOTUNE_VERBOSE=1 prints every trial and the choice to stderr.  Tile configurations: 128 x 256 with the stage count that
-// fits (2 for the split modes, 4 otherwise) and 128 x 128 with more stages (3 / 6): the wide tile
-// reads each A panel half as often, the narrow one keeps a deeper copy pipeline.  Small problems,
-// launches that accumulate or are being captured, and TDSCHA_AUTOTUNE=0 use the wide tile in the
-// m-fastest order; TDSCHA_TILE_N (256 | 128) and TDSCHA_GROUP_M fix the choice.
-static std::map<TuneKey, std::pair<int, int>> g_tune_cfg;
+template <bool TF32, int NPROD>
+static int prepare(const GemmOperands &op, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
+                   long long ldd, cudaStream_t st, unsigned *err, unsigned *counter, int stall, int sms, Prepared *out) {
+    const int c = sh.cap <= 64 ? 64 : (sh.cap <= 128 ? 128 : 256);
+    // half stages where full ones would leave the ring two deep
+    constexpr int NOPS = NPROD == 3 ? 2 : 1;
+    const int room = SMEM_MAX - SMEM_FIXED - (sh.swap ? 0 : EPI_STAGING);
+    const bool half = c == 256 && room / (NOPS * 128 * (sh.p_rows + pl.q_rows)) < 3;
+#define TD_PREP(C, SW, KBY) prepare_cfg<C, TF32, NPROD, SW, KBY>(op, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, out)
+    if (sh.swap) {
+        if (half) return TD_PREP(256, true, 64);
+        return c == 64 ? TD_PREP(64, true, 128) : (c == 128 ? TD_PREP(128, true, 128) : TD_PREP(256, true, 128));
+    }
+    if (half) return TD_PREP(256, false, 64);
+    return c == 64 ? TD_PREP(64, false, 128) : (c == 128 ? TD_PREP(128, false, 128) : TD_PREP(256, false, 128));
+#undef TD_PREP
+}
 
-static int choose(int tf32, int nprod, int M, int N, int K, unsigned long long shape, const Prepared *cfgs, int ncfg,
-                  cudaStream_t st, bool allow_trials, int *cfg_out, int *gm_out) {
-    int dev = 0, sms = 148;
-    TD_CUDA(cudaGetDevice(&dev));
-    TD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    int forced_cfg = -1;
-    if (const char *env = getenv("TDSCHA_TILE_N")) forced_cfg = atoi(env) == 128 ? 1 : 0;
-    const char *env_gm = getenv("TDSCHA_GROUP_M");
-    if (forced_cfg >= 0 || env_gm) {
-        const int c = forced_cfg >= 0 ? std::min(forced_cfg, ncfg - 1) : 0;
-        *cfg_out = c;
-        *gm_out = env_gm ? std::max(1, std::min(cfgs[c].num_m, atoi(env_gm))) : cfgs[c].num_m;
+// ---- tile-order autotuner ---------------------------------------------------------------------------
+// On the first call for a (format, products, M, N, K) with many tiles (8 per SM and more) and more than
+// 24 P tiles, the launcher times the tile-group sizes on the caller's stream and remembers the winner
+// (with fewer P tiles every order is within 3 %: the class contractions of 768 to 3072 rows):
+// the candidates run in turn, twice round (every run writes the same D), and each keeps its faster run,
+// so that the clock drift of a power-capped GPU over the trials does not favour the candidates timed
+// first.  TDSCHA_AUTOTUNE_VERBOSE=1 prints every trial and the choice to stderr.  Swapped launches,
+// small problems, launches that accumulate or are being captured, and TDSCHA_AUTOTUNE=0 use the
+// P-fastest order; TDSCHA_GROUP_M fixes the choice.
+static std::map<TuneKey, int> g_tune_gp;
+
+static int choose_order(const TuneKey &key, const Prepared &cfg, int sms, cudaStream_t st, bool allow_trials, int *gp_out) {
+    *gp_out = cfg.shape.swap ? 1 : cfg.num_p;
+    if (cfg.shape.swap) return 0;
+    if (const char *env_gm = getenv("TDSCHA_GROUP_M")) {
+        *gp_out = std::max(1, std::min(cfg.num_p, atoi(env_gm)));
         return 0;
     }
-    const TuneKey key{tf32, nprod, M, N, K, dev, shape};
+    if (cfg.tiles < 8LL * sms || cfg.num_p <= 24) return 0;
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
-        auto it = g_tune_cfg.find(key);
-        if (it != g_tune_cfg.end()) { *cfg_out = it->second.first; *gm_out = it->second.second; return 0; }
+        auto it = g_tune_gp.find(key);
+        if (it != g_tune_gp.end()) { *gp_out = it->second; return 0; }
     }
     const char *env = getenv("TDSCHA_AUTOTUNE");
-    const bool enabled = allow_trials && !(env && atoi(env) == 0);
-    int best_c = 0, best_gm = cfgs[0].num_m;
+    if (!allow_trials || (env && atoi(env) == 0)) return 0;
     const char *env_v = getenv("TDSCHA_AUTOTUNE_VERBOSE");
     const bool verbose = env_v && atoi(env_v) == 1;
-    if (enabled && cfgs[0].tiles >= 8LL * sms) {
-        std::vector<std::pair<int, int>> cands;   // (configuration, tile-group size)
-        for (int c = 0; c < ncfg; ++c) {
-            const int num_m = cfgs[c].num_m;
-            const int cand_all[] = {num_m, 48, 24, 12, 6};
-            for (int ci = 0; ci < 5; ++ci) {
-                const int cand = cand_all[ci];
-                bool dup = cand > num_m;
-                for (int cj = 0; cj < ci; ++cj) dup = dup || cand_all[cj] == cand;
-                if (!dup) cands.push_back({c, cand});
-            }
+    std::vector<int> cands;
+    for (int cand : {cfg.num_p, 48, 24, 12, 6})
+        if (cand <= cfg.num_p && std::find(cands.begin(), cands.end(), cand) == cands.end()) cands.push_back(cand);
+    cudaEvent_t e0, e1;
+    TD_CUDA(cudaEventCreate(&e0));
+    TD_CUDA(cudaEventCreate(&e1));
+    std::vector<float> t_min(cands.size(), 1e30f);
+    for (int round = 0; round < 2 && cands.size() > 1; ++round)
+        for (size_t i = 0; i < cands.size(); ++i) {
+            TD_CUDA(cudaEventRecord(e0, st));
+            cfg.launch(cands[i]);
+            TD_CUDA(cudaGetLastError());
+            TD_CUDA(cudaEventRecord(e1, st));
+            TD_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            TD_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            t_min[i] = std::min(t_min[i], ms);
+            if (verbose)
+                fprintf(stderr, "[tc autotune] M=%d N=%d K=%d nprod=%d tile_n=%d group=%d round %d: %.3f ms\n", key.M, key.N, key.K,
+                        key.nprod, cfg.shape.cap, cands[i], round, ms);
         }
-        cudaEvent_t e0, e1;
-        TD_CUDA(cudaEventCreate(&e0));
-        TD_CUDA(cudaEventCreate(&e1));
-        std::vector<float> t_min(cands.size(), 1e30f);
-        for (int round = 0; round < 2; ++round)
-            for (size_t i = 0; i < cands.size(); ++i) {
-                TD_CUDA(cudaEventRecord(e0, st));
-                cfgs[cands[i].first].launch(cands[i].second);
-                TD_CUDA(cudaGetLastError());
-                TD_CUDA(cudaEventRecord(e1, st));
-                TD_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                TD_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                t_min[i] = std::min(t_min[i], ms);
-                if (verbose)
-                    fprintf(stderr, "[tc autotune] M=%d N=%d K=%d nprod=%d tile_n=%d group_m=%d round %d: %.3f ms\n", M, N, K,
-                            nprod, cfgs[cands[i].first].bn, cands[i].second, round, ms);
-            }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        size_t bi = 0;
-        for (size_t i = 1; i < cands.size(); ++i)
-            if (t_min[i] < t_min[bi]) bi = i;
-        best_c = cands[bi].first;
-        best_gm = cands[bi].second;
-    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    size_t bi = 0;
+    for (size_t i = 1; i < cands.size(); ++i)
+        if (t_min[i] < t_min[bi]) bi = i;
     if (verbose)
-        fprintf(stderr, "[tc autotune] M=%d N=%d K=%d nprod=%d -> tile_n=%d group_m=%d\n", M, N, K, nprod, cfgs[best_c].bn,
-                best_gm);
+        fprintf(stderr, "[tc autotune] M=%d N=%d K=%d nprod=%d -> tile_n=%d group=%d\n", key.M, key.N, key.K, key.nprod,
+                cfg.shape.cap, cands[bi]);
     std::lock_guard<std::mutex> lock(g_tune_mutex);
-    if (allow_trials) g_tune_cfg[key] = {best_c, best_gm};
-    *cfg_out = best_c;
-    *gm_out = best_gm;
+    g_tune_gp[key] = cands[bi];
+    *gp_out = cands[bi];
     return 0;
+}
+
+// The tile shape with the least estimated time (plan_tiles), remembered per problem shape.
+// TDSCHA_TILE_N (256 | 128 | 64) forces tiles of that many output columns with A on the 128-row side.
+static std::map<std::pair<TuneKey, int>, std::pair<TileShape, TilePlan>> g_tune_shape;
+
+static TileShape choose_shape(const Problem &pb, size_t g0, size_t g1, const TuneKey &key, int kelems, int nprod, int drain, int sms,
+                              bool stall, TilePlan *plan) {
+    TileShape best;
+    const char *env = getenv("TDSCHA_TILE_N");
+    if (env || stall) {   // abort-path test: the wide tile
+        if (env && (atoi(env) == 128 || atoi(env) == 64)) best.cap = atoi(env);
+        *plan = plan_tiles(pb, g0, g1, best, kelems, nprod, drain, sms);
+        return best;
+    }
+    std::lock_guard<std::mutex> lock(g_tune_mutex);
+    auto it = g_tune_shape.find({key, drain});
+    if (it != g_tune_shape.end()) {
+        *plan = it->second.second;
+        return it->second.first;
+    }
+    plan->cycles = 1e300;
+    for (int swap = 0; swap < 2; ++swap)
+        for (int cap : {256, 192, 128, 96, 64, 48, 32, 16})
+            for (int p_rows : {128, 64}) {
+                const TileShape sh{swap != 0, cap, p_rows};
+                const TilePlan pl = plan_tiles(pb, g0, g1, sh, kelems, nprod, drain, sms);
+                if (pl.cycles < plan->cycles) { *plan = pl; best = sh; }
+            }
+    const char *env_v = getenv("TDSCHA_AUTOTUNE_VERBOSE");
+    if (env_v && atoi(env_v) == 1)
+        fprintf(stderr, "[tc shape] %zu groups, first M=%d N=%d K=%d: %s cap %d, %d P rows, q box %d, %lld tiles, %.0f cycles\n", g1 - g0,
+                pb.groups[g0].M, pb.groups[g0].N, pb.groups[g0].K, best.swap ? "swapped" : "normal", best.cap, best.p_rows,
+                plan->q_box, plan->tiles, plan->cycles);
+    g_tune_shape[{key, drain}] = {best, *plan};
+    return best;
 }
 
 template <bool TF32, int NPROD>
 static int launch_tuned(const GemmOperands &op, const Problem &pb, float *D, long long ldd, cudaStream_t st, unsigned *err) {
-    constexpr int S_WIDE = NPROD == 3 ? 2 : 4, S_NARROW = NPROD == 3 ? 3 : 6, S_THIN = NPROD == 3 ? 4 : 8;
-    int dev = 0;
+    int dev = 0, sms = 148;
     TD_CUDA(cudaGetDevice(&dev));
+    TD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     TD_CUDA(cudaStreamIsCapturing(st, &cap));
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     unsigned *counter = nullptr;
     if (tile_sync_budget_ns() > 0) TD_TRY(tile_sync_counter(dev, st, capturing, &counter));
     const int stall = g_stall_next.exchange(0);
+    const int drain = op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD);
     for (size_t g0 = 0; g0 < pb.groups.size(); g0 += MAX_GROUPS) {
         const size_t g1 = std::min(pb.groups.size(), g0 + MAX_GROUPS);
-        Prepared cfgs[3];
-        TD_TRY((prepare_cfg<256, S_WIDE, TF32, NPROD>(op, pb, g0, g1, D, ldd, st, err, counter, stall, &cfgs[0])));
-        TD_TRY((prepare_cfg<128, S_NARROW, TF32, NPROD>(op, pb, g0, g1, D, ldd, st, err, counter, stall, &cfgs[1])));
-        // outputs at most 64 columns wide in every group (the per-class mode-column contractions): the
-        // 128 x 64 tile, whose shorter B rows leave room for a deeper A stream, and no wasted MMA columns
-        bool thin = true;
-        for (size_t i = g0; i < g1; ++i) thin = thin && pb.groups[i].N <= 64;
-        const char *env_tn = getenv("TDSCHA_TILE_N");
-        if (env_tn) thin = thin && atoi(env_tn) == 64;
-        if (thin) TD_TRY((prepare_cfg<64, S_THIN, TF32, NPROD>(op, pb, g0, g1, D, ldd, st, err, counter, stall, &cfgs[2])));
         // tuning key: the one problem's shape, or the groups' shapes hashed (FNV-1a)
-        int kM = pb.groups[g0].M, kN = pb.groups[g0].N, kK = pb.groups[g0].K;
-        unsigned long long shape = 0;
+        TuneKey key{TF32 ? 1 : 0, NPROD, pb.groups[g0].M, pb.groups[g0].N, pb.groups[g0].K, dev, 0ull};
         if (g1 - g0 > 1) {
-            shape = 1469598103934665603ull;
+            key.shape = 1469598103934665603ull;
             for (size_t i = g0; i < g1; ++i)
                 for (long long v : {(long long)pb.groups[i].M, (long long)pb.groups[i].N, (long long)pb.groups[i].K}) {
-                    shape ^= (unsigned long long)v;
-                    shape *= 1099511628211ull;
+                    key.shape ^= (unsigned long long)v;
+                    key.shape *= 1099511628211ull;
                 }
-            kM = (int)(g1 - g0);
+            key.M = (int)(g1 - g0);
         }
-        int c = 0, gm = cfgs[0].num_m;
-        if (thin && !stall) {
-            c = 2;
-            gm = cfgs[2].num_m;
-        } else if (!stall) {   // abort-path test: one launch of the wide tile, no tuning trials
-            // trial runs write D, so an accumulating launch only reuses a choice tuned earlier (and a
-            // launch being captured into a CUDA graph runs nothing, so it cannot time trials)
-            TD_TRY(choose(TF32 ? 1 : 0, NPROD, kM, kN, kK, shape, cfgs, 2, st, !op.accumulate && !capturing, &c, &gm));
-        }
-        cfgs[c].launch(gm);
+        TilePlan pl;
+        const TileShape sh = choose_shape(pb, g0, g1, key, KBlock<TF32, 128>::ELEMS, NPROD, drain, sms, stall != 0, &pl);
+        Prepared cfg;
+        TD_TRY((prepare<TF32, NPROD>(op, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, &cfg)));
+        int gp = cfg.num_p;
+        // trial runs write D, so an accumulating launch only reuses a choice tuned earlier (and a launch
+        // being captured into a CUDA graph runs nothing, so it cannot time trials); the abort-path
+        // test runs one launch without trials
+        if (!stall) TD_TRY(choose_order(key, cfg, sms, st, !op.accumulate && !capturing, &gp));
+        cfg.launch(gp);
         TD_CUDA(cudaGetLastError());
     }
     return 0;
