@@ -43,7 +43,7 @@ __device__ __forceinline__ void unpair(long long p, int n, int &mu, int &nu) {
 }
 
 // ---- prologue: (R1, Upsilon^(1)) of each vector ----------------------------------------------
-__global__ void prologue_kernel(int nb, int n, long long len, const double *__restrict__ psi, const int *__restrict__ transpose,
+__global__ void prologue_kernel(int nb, int n, long long len, const double *__restrict__ psi, TransposeFlags transpose,
                                 const double *__restrict__ w, double T, int use_wigner, double *R, double *Ys) {
     const long long P = (long long)n * (n + 1) / 2;
     const long long total = (long long)nb * P;
@@ -87,7 +87,7 @@ __global__ void prologue_kernel(int nb, int n, long long len, const double *__re
 }
 
 // ---- epilogue: L1 + anharmonic packing, reverse, shift -----------------------------------------
-__global__ void epilogue_kernel(int nb, int n, long long len, const double *__restrict__ psi, const int *__restrict__ transpose,
+__global__ void epilogue_kernel(int nb, int n, long long len, const double *__restrict__ psi, TransposeFlags transpose,
                                 const double *__restrict__ w, double T, tdscha_apply_opts o, const double *__restrict__ fav,
                                 const double *__restrict__ dav, double *__restrict__ out) {
     const long long P = (long long)n * (n + 1) / 2;
@@ -165,20 +165,17 @@ int apply_full_L_device(tdscha_ensemble *e, int nb, const double *psi, const int
                         int precision, double *out, cudaStream_t st, void *scratch, size_t scratch_bytes) {
     TD_CHECK(e && psi && out && transpose_h && scratch, TDSCHA_EINVAL, "NULL argument");
     TD_CHECK(nb > 0 && nb <= 64, TDSCHA_EINVAL, "1..64 vectors per apply call (got %d)", nb);
-    TD_CHECK(scratch_bytes > 256, TDSCHA_EINVAL, "apply scratch too small");
-    // scratch: transpose flags (nb ints, 256 bytes), then the work of apply_full_L_device_flags
-    uint8_t *s = static_cast<uint8_t *>(scratch);
-    int *tr_d = reinterpret_cast<int *>(s);
-    TD_CUDA(cudaMemcpyAsync(tr_d, transpose_h, nb * sizeof(int), cudaMemcpyHostToDevice, st));
-    return apply_full_L_device_flags(e, nb, psi, tr_d, opts, precision, out, st, reinterpret_cast<double *>(s + 256),
-                                     scratch_bytes - 256);
+    TransposeFlags tr;
+    for (int k = 0; k < nb; ++k)
+        if (transpose_h[k]) tr.mask |= 1ull << k;
+    return apply_full_L_device_flags(e, nb, psi, tr, opts, precision, out, st, static_cast<double *>(scratch), scratch_bytes);
 }
 
-// apply_full_L with the transpose flags already on the device (no host transfer: graph-capturable);
+// apply_full_L without a host transfer (graph-capturable);
 // work: R (nb n), Ys (nb n^2), f (nb n), D (nb n^2) doubles.
-int apply_full_L_device_flags(tdscha_ensemble *e, int nb, const double *psi, const int *tr_d, const tdscha_apply_opts *opts,
+int apply_full_L_device_flags(tdscha_ensemble *e, int nb, const double *psi, TransposeFlags tr, const tdscha_apply_opts *opts,
                               int precision, double *out, cudaStream_t st, double *work, size_t work_bytes) {
-    TD_CHECK(e && psi && out && tr_d && work, TDSCHA_EINVAL, "NULL argument");
+    TD_CHECK(e && psi && out && work, TDSCHA_EINVAL, "NULL argument");
     TD_CHECK(nb > 0 && nb <= 64, TDSCHA_EINVAL, "1..64 vectors per apply call (got %d)", nb);
     tdscha_apply_opts o{0, 0, 0, 0, 0, 0.0};
     if (opts) o = *opts;
@@ -192,11 +189,11 @@ int apply_full_L_device_flags(tdscha_ensemble *e, int nb, const double *psi, con
     double *dav = fav + (size_t)nb * n;
     e->prof.launches[ST_OTHER] += o.ignore_v3 ? 1 : 2;
     if (!o.ignore_v3) {
-        prologue_kernel<<<grid_for((long long)nb * P), 256, 0, st>>>(nb, n, len, psi, tr_d, e->w, e->T, o.use_wigner, R, Ys);
+        prologue_kernel<<<grid_for((long long)nb * P), 256, 0, st>>>(nb, n, len, psi, tr, e->w, e->T, o.use_wigner, R, Ys);
         TD_CUDA(cudaGetLastError());
         TD_TRY(perturb_average_device(e, nb, R, Ys, o.ignore_v4 ? 0 : 1, precision, fav, dav, st));
     }
-    epilogue_kernel<<<grid_for((long long)nb * len), 256, 0, st>>>(nb, n, len, psi, tr_d, e->w, e->T, o, fav, dav, out);
+    epilogue_kernel<<<grid_for((long long)nb * len), 256, 0, st>>>(nb, n, len, psi, tr, e->w, e->T, o, fav, dav, out);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
@@ -211,7 +208,7 @@ int apply_prologue_device(tdscha_ensemble *e, int nb, const double *psi, const i
     const int n = e->n;
     const long long P = (long long)n * (n + 1) / 2;
     e->prof.launches[ST_OTHER] += 1;
-    prologue_kernel<<<grid_for((long long)nb * P), 256, 0, st>>>(nb, n, n + 2 * P, psi, tr_d, e->w, e->T, o.use_wigner, R, Ys);
+    prologue_kernel<<<grid_for((long long)nb * P), 256, 0, st>>>(nb, n, n + 2 * P, psi, TransposeFlags{tr_d, 0ull}, e->w, e->T, o.use_wigner, R, Ys);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
@@ -225,14 +222,14 @@ int apply_epilogue_device(tdscha_ensemble *e, int nb, const double *psi, const i
     const int n = e->n;
     const long long len = n + (long long)n * (n + 1);
     e->prof.launches[ST_OTHER] += 1;
-    epilogue_kernel<<<grid_for((long long)nb * len), 256, 0, st>>>(nb, n, len, psi, tr_d, e->w, e->T, o, fav, dav, out);
+    epilogue_kernel<<<grid_for((long long)nb * len), 256, 0, st>>>(nb, n, len, psi, TransposeFlags{tr_d, 0ull}, e->w, e->T, o, fav, dav, out);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
 
 size_t apply_scratch_bytes(const tdscha_ensemble *e, int nb) {
     const size_t n = e->n;
-    return 256 + (size_t)nb * (2 * n + 2 * n * n) * sizeof(double);
+    return (size_t)nb * (2 * n + 2 * n * n) * sizeof(double);
 }
 
 // ---- bi-conjugate Lanczos step ----------------------------------------------------------------

@@ -8,9 +8,17 @@
 
 namespace tdscha {
 
+// Transpose flag of each vector of a call: a device array, or (ptr null, at most 64 vectors) one bit
+// per vector in the kernel's arguments, which needs no copy to the device.
+struct TransposeFlags {
+    const int *ptr = nullptr;
+    unsigned long long mask = 0;
+    __device__ __forceinline__ int operator[](int k) const { return ptr ? ptr[k] : (int)((mask >> k) & 1ull); }
+};
+
 int apply_full_L_device(tdscha_ensemble *e, int nb, const double *psi, const int *transpose_h, const tdscha_apply_opts *opts,
                         int precision, double *out, cudaStream_t st, void *scratch, size_t scratch_bytes);
-int apply_full_L_device_flags(tdscha_ensemble *e, int nb, const double *psi, const int *tr_d, const tdscha_apply_opts *opts,
+int apply_full_L_device_flags(tdscha_ensemble *e, int nb, const double *psi, TransposeFlags tr, const tdscha_apply_opts *opts,
                               int precision, double *out, cudaStream_t st, double *work, size_t work_bytes);
 size_t apply_scratch_bytes(const tdscha_ensemble *e, int nb);
 int apply_prologue_device(tdscha_ensemble *e, int nb, const double *psi, const int *tr_d, const tdscha_apply_opts *opts,

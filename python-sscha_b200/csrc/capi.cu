@@ -55,10 +55,21 @@ static int scratch_get(int slot, size_t bytes, cudaStream_t st, void **out) {
 // Per-call reading of the error word (tdscha_set_error_check); off: tdscha_check_errors reads it.
 static std::atomic<int> g_check_per_call{1};
 
+// The word lands in page-locked memory, one word per host thread (kept for the thread's life): a copy
+// to pageable memory goes through the driver's staging buffer.
+struct PinnedWord {
+    unsigned *p = nullptr;
+    ~PinnedWord() {
+        if (p) cudaFreeHost(p);
+    }
+};
+static thread_local PinnedWord g_err_word;
+
 static int read_err_word(tdscha_ensemble *e, cudaStream_t st) {
-    unsigned h = 0;
-    TD_CUDA(cudaMemcpyAsync(&h, e->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    if (!g_err_word.p) TD_CUDA(cudaHostAlloc(&g_err_word.p, sizeof(unsigned), cudaHostAllocPortable));
+    TD_CUDA(cudaMemcpyAsync(g_err_word.p, e->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     TD_CUDA(cudaStreamSynchronize(st));
+    const unsigned h = *g_err_word.p;
     if (h) {
         cudaMemsetAsync(e->d_err, 0, sizeof(unsigned), st);
         set_error("a tensor-core kernel hit its bounded-wait limit and aborted (error word 0x%x)", h);

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdarg>
+#include <atomic>
 
 #include "tdscha_b200.h"
 
@@ -36,6 +37,19 @@ void clear_error();
         int rc_ = (expr);                                                                      \
         if (rc_ != 0) return rc_;                                                              \
     } while (0)
+
+// Allows a kernel `bytes` of dynamic shared memory: one driver call per kernel and device, not one per
+// launch (the attribute outlives the call; `bytes` is the most the kernel is ever launched with).
+template <auto Kernel>
+inline int allow_smem(int bytes) {
+    static std::atomic<unsigned long long> done{0};   // one bit per device
+    int dev = 0;
+    TD_CUDA(cudaGetDevice(&dev));
+    if (dev < 64 && ((done.load() >> dev) & 1ull)) return 0;
+    TD_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (dev < 64) done.fetch_or(1ull << dev);
+    return 0;
+}
 
 constexpr double RY_TO_K = 157887.32400374097;  // CModules/LanczosFunctions.h:9
 

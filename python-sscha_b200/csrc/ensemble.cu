@@ -765,6 +765,11 @@ static bool fused_cd_enabled() {
     return env && atoi(env) == 1;
 }
 
+// An averages call whose operands are built and whose workspace holds all of its rows plans nothing: the
+// device memory query behind the chunking takes 70 us and waits on a driver lock (milliseconds when
+// other processes use the machine).  Forced chunk sizes always go through the planning.
+static bool chunks_forced() { return getenv("TDSCHA_CONFIG_CHUNK") || getenv("TDSCHA_SYM_CHUNK"); }
+
 static bool use_freq_path(const tdscha_ensemble *e, Format fmt) {
     return e->freq && e->cosets && cosets_enabled() && freq_enabled() && !(fmt == FMT_BF16 && sym_umma_enabled());
 }
@@ -880,6 +885,12 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
             TD_CHECK(e->fops[fmt].built && (e->fops[fmt].has_lo || !lo), TDSCHA_EINVAL, "operands released since the plan");
             co = e->fops[fmt];
         }
+    } else if (!chunks_forced() && e->fops[fmt].built && (e->fops[fmt].has_lo || !lo) &&
+               e->ws.bytes >= freq_ws_layout(e, nb, (int)round_up(n_cos, Jf), nf_total, fmt, lo, e->N).total) {
+        // everything in one pass, with the operands and the workspace of earlier calls: nothing to plan
+        ncj = (int)round_up(n_cos, Jf);
+        co = e->fops[fmt];
+        e->plan = AvgPlan{true, nb, (int)fmt, lo, true, true, false, Nc, ncj * sub};
     } else {
         size_t free_b = 0, tot_b = 0;
         TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
@@ -1127,6 +1138,12 @@ int perturb_average_device(tdscha_ensemble *e, int nb, const double *R1, const d
             TD_CHECK(e->ops[fmt].built && (e->ops[fmt].has_lo || !lo), TDSCHA_EINVAL, "operands released since the plan");
             co = e->ops[fmt];
         }
+    } else if (const int Jall = (int)round_up(e->N_sym, unit);
+               !chunks_forced() && e->ops[fmt].built && (e->ops[fmt].has_lo || !lo) &&
+               e->ws.bytes >= layout(e, nb, Jall, nf_total, fmt, lo, e->N, use_cos ? Jall / sub : 0).total) {
+        Jc = Jall;
+        co = e->ops[fmt];
+        e->plan = AvgPlan{true, nb, (int)fmt, lo, use_cos, false, false, Nc, Jc};
     } else {
         // Configuration chunk: all configurations when their operands fit in half of the free memory
         // (then they stay resident between calls), else chunks of Nc whose operands are rebuilt from
@@ -1559,12 +1576,15 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
     const size_t fixed = 4 * ((size_t)N * Kp + 2 * (size_t)N * np) + 8 * ((size_t)N + (size_t)nb * n + (size_t)nb * n * n) +
                          16 * 256;
     const size_t per_row = es * nh * (4 * (size_t)Kp + 4 * (size_t)np + 4 * (size_t)N) + 4 * 4 * (size_t)ld1 + 8 * (size_t)N;
-    size_t free_b = 0, tot_b = 0;
-    TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
-    const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
-    TD_CHECK(budget > fixed + per_row * (nb + 64), TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
-    int Jc = (int)std::min<long long>(e->N_sym, (long long)((budget - fixed) / per_row - 64) / nb);
-    Jc = std::max(1, Jc);
+    int Jc = e->N_sym;
+    if (e->vjp_ws.bytes < fixed + per_row * (size_t)round_up((long long)nb * Jc, 64) + 64 * 256) {
+        size_t free_b = 0, tot_b = 0;
+        TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+        const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
+        TD_CHECK(budget > fixed + per_row * (nb + 64), TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
+        Jc = (int)std::min<long long>(e->N_sym, (long long)((budget - fixed) / per_row - 64) / nb);
+        Jc = std::max(1, Jc);
+    }
     const long long Mmax = (long long)nb * Jc, Mpmax = round_up(Mmax, 64);
     const size_t need = fixed + per_row * (size_t)Mpmax + 64 * 256;
     if (e->vjp_ws.bytes < need) {
@@ -1693,12 +1713,14 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
         b += 8 * rows * (size_t)N;                                           // BR
         return b + 32 * 256;
     };
-    size_t free_b = 0, tot_b = 0;
-    TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
-    const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
-    TD_CHECK(budget > fixed + per_chunk(1), TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
     int ncj = n_cos;
-    while (ncj > 1 && fixed + per_chunk(ncj) > budget) ncj = (ncj + 1) / 2;
+    if (e->vjp_ws.bytes < fixed + per_chunk(ncj)) {   // no query when the workspace of an earlier call holds everything
+        size_t free_b = 0, tot_b = 0;
+        TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+        const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
+        TD_CHECK(budget > fixed + per_chunk(1), TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
+        while (ncj > 1 && fixed + per_chunk(ncj) > budget) ncj = (ncj + 1) / 2;
+    }
     const size_t need = fixed + per_chunk(ncj);
     if (e->vjp_ws.bytes < need) {
         if (e->vjp_ws.base) { TD_CUDA(cudaDeviceSynchronize()); cudaFree(e->vjp_ws.base); e->vjp_ws = Workspace(); }
@@ -1890,12 +1912,15 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
     // persistent buffers, then per-chunk rows (M = nb * Jc)
     const size_t fixed = 8 * ((size_t)N * e->Kp + 2 * (size_t)N * e->np + N + (size_t)nb * n + (size_t)nb * n * n) + 8 * 256;
     const size_t per_row = 8 * (2 * (size_t)e->Kp + 2 * (size_t)e->np + 4 * (size_t)ld1 + 5 * (size_t)N);
-    size_t free_b = 0, tot_b = 0;
-    TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
-    const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
-    TD_CHECK(budget > fixed + per_row * nb, TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
-    int Jc = std::min<long long>(e->N_sym, (long long)((budget - fixed) / (per_row * nb)));
-    Jc = std::max(1, Jc);
+    int Jc = e->N_sym;
+    if (e->vjp_ws.bytes < fixed + per_row * (size_t)nb * Jc + 16 * 256) {
+        size_t free_b = 0, tot_b = 0;
+        TD_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+        const size_t budget = std::max<size_t>((size_t)1 << 30, (size_t)((free_b + e->vjp_ws.bytes) * 0.5));
+        TD_CHECK(budget > fixed + per_row * nb, TDSCHA_ENOMEM, "not enough device memory for the averages' VJP");
+        Jc = std::min<long long>(e->N_sym, (long long)((budget - fixed) / (per_row * nb)));
+        Jc = std::max(1, Jc);
+    }
     const size_t need = fixed + per_row * (size_t)nb * Jc + 16 * 256;
     if (e->vjp_ws.bytes < need) {
         if (e->vjp_ws.base) { TD_CUDA(cudaDeviceSynchronize()); cudaFree(e->vjp_ws.base); e->vjp_ws = Workspace(); }

@@ -510,8 +510,8 @@ int build_Vq_cols(const FreqTables &t, const double *XGT, long long ldT, int n, 
     TD_CHECK(t.Kq % COLS == 0 && N2pc % 64 == 0 && ceil_div(N2pc, 256) <= 65535, TDSCHA_EINVAL, "operand build: %lld x %d",
              N2pc, t.Kq);
     const size_t smem = (size_t)2 * COLS * 257 * sizeof(T);
-    auto kern = build_Vq_cols_kernel<T>;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = build_Vq_cols_kernel<T>;
+    TD_TRY(allow_smem<kern>((int)smem));
     const dim3 grid((unsigned)(t.Kq / COLS), (unsigned)ceil_div(N2pc, 256));
     kern<<<grid, 256, smem, st>>>(XGT, ldT, n, Nc, N2pc, t.Kq, t.pc_mu0, t.pc_nu0, t.pc_mu1, t.pc_nu1, t.pc_c0, t.pc_c1, fmt,
                                   static_cast<T *>(V_hi), static_cast<T *>(V_lo), static_cast<T *>(VT_hi), static_cast<T *>(VT_lo));

@@ -87,7 +87,7 @@ struct SysWork {
     size_t apply_bytes = 0;
     double *lz = nullptr;
     size_t lz_bytes = 0;
-    int *tr = nullptr;          // (2 nc) transpose flags: nc zeros, nc ones
+    TransposeFlags tr;          // of the 2 nc vectors: L for q, the transpose for p
     int *counter = nullptr;
     int *done = nullptr;        // (nc) chain ended by a breakdown
     cudaStream_t stream = nullptr;
@@ -106,7 +106,6 @@ struct RunState {
             cudaFree(s.sc_out);
             cudaFree(s.apply_work);
             cudaFree(s.lz);
-            cudaFree(s.tr);
             cudaFree(s.counter);
             cudaFree(s.done);
             if (s.joined) cudaEventDestroy(s.joined);
@@ -214,13 +213,10 @@ int lanczos_run_device(int ns, const tdscha_run_system *sys, int n_steps, int us
         TD_CUDA(cudaMalloc(&w.apply_work, w.apply_bytes));
         w.lz_bytes = lanczos_scratch_bytes(nc);
         TD_CUDA(cudaMalloc(&w.lz, w.lz_bytes));
-        TD_CUDA(cudaMalloc(&w.tr, nb * sizeof(int)));
         TD_CUDA(cudaMalloc(&w.counter, sizeof(int)));
         TD_CUDA(cudaMalloc(&w.done, nc * sizeof(int)));
         TD_CUDA(cudaMemset(w.done, 0, nc * sizeof(int)));
-        std::vector<int> tr(nb, 0);
-        for (int c = nc; c < nb; ++c) tr[c] = 1;
-        TD_CUDA(cudaMemcpy(w.tr, tr.data(), nb * sizeof(int), cudaMemcpyHostToDevice));
+        for (int c = nc; c < nb; ++c) w.tr.mask |= 1ull << c;
         TD_CUDA(cudaMemset(w.counter, 0, sizeof(int)));
     }
     // profiling events cannot be read back from graph replays: off for the run

@@ -231,8 +231,8 @@ static int launch_transform(const SymTables &t, const PairClasses &pc, int nb, i
     if (!pc.count[MT]) return 0;
     constexpr int JT = 8;
     const size_t smem = 4 * (size_t)(16 * MT) * (16 * MT) * sizeof(T);
-    auto kern = transform_kernel<T, MT>;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = transform_kernel<T, MT>;
+    TD_TRY(allow_smem<kern>((int)smem));
     dim3 grid((unsigned)pc.count[MT], (unsigned)ceil_div(nj, JT), (unsigned)nb);
     kern<<<grid, SYM_THREADS, smem, st>>>(t, pc.b[MT], pc.c[MT], nj, j0, JT, Ys, R1, ups, Kp, np, fmt, B1_hi, B1_lo, r1_hi, r1_lo);
     TD_CUDA(cudaGetLastError());
@@ -273,8 +273,8 @@ static int launch_fold(const SymTables &t, const PairClasses &pc, int nb, int nj
                        long long ldz, const AccT *F, long long ldf, const double *ups, double *partD, double *partF, cudaStream_t st) {
     if (!pc.count[MT]) return 0;
     const size_t smem = 4 * (size_t)(16 * MT) * (16 * MT) * sizeof(T);
-    auto kern = fold_kernel<T, AccT, MT>;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = fold_kernel<T, AccT, MT>;
+    TD_TRY(allow_smem<kern>((int)smem));
     dim3 grid((unsigned)pc.count[MT], (unsigned)ceil_div(nj, Jf), (unsigned)nb);
     kern<<<grid, SYM_THREADS, smem, st>>>(t, pc.b[MT], pc.c[MT], Z, ldz, F, ldf, ups, nj, j0, Jf, nf_total, partD, partF);
     TD_CUDA(cudaGetLastError());

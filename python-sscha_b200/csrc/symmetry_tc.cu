@@ -555,7 +555,8 @@ int launch_transform_tc(const SymTables &t, const PairClasses &pc, int nb, int n
     const bool lean = !(env && atoi(env) == 0);
     auto kern = lean ? transform_tc_lean_kernel<MT> : transform_tc_kernel<MT>;
     const size_t smem = lean ? S::SMEM / 2 : S::SMEM;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (lean) TD_TRY(allow_smem<transform_tc_lean_kernel<MT>>((int)smem));
+    else TD_TRY(allow_smem<transform_tc_kernel<MT>>((int)smem));
     dim3 grid((unsigned)pc.count[MT], (unsigned)ceil_div(nj, JT), (unsigned)nb);
     kern<<<grid, S::THREADS, smem, st>>>(t, pc.b[MT], pc.c[MT], nj, j0, JT, Ys, R1, ups, Kp, np, fmt, B1_hi, B1_lo, r1_hi, r1_lo);
     TD_CUDA(cudaGetLastError());
@@ -574,7 +575,8 @@ int launch_fold_tc(const SymTables &t, const PairClasses &pc, int nb, int nj, in
     auto kern = lean ? fold_tc_lean_kernel<MT> : fold_tc_kernel<MT>;
     const size_t smem = lean ? S::SMEM / 2 : S::SMEM;
     const int threads = lean ? lean_fold_threads(MT) : S::THREADS;
-    TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (lean) TD_TRY(allow_smem<fold_tc_lean_kernel<MT>>((int)smem));
+    else TD_TRY(allow_smem<fold_tc_kernel<MT>>((int)smem));
     dim3 grid((unsigned)pc.count[MT], (unsigned)ceil_div(nj, Jf), (unsigned)nb);
     kern<<<grid, threads, smem, st>>>(t, pc.b[MT], pc.c[MT], Z, ldz, F, ldf, ups, nj, j0, Jf, nf_total, partD, partF);
     TD_CUDA(cudaGetLastError());

@@ -753,14 +753,8 @@ static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, siz
     }
     TD_CHECK(tiles < (1LL << 31), TDSCHA_EINVAL, "tc::gemm: %lld tiles exceed the schedule", tiles);
     gt.total_tiles = (int)tiles;
-    auto kern = tc_gemm_kernel<MAXC, TF32, NPROD, SWAP, KBYTES>;
-    static std::atomic<unsigned long long> attr_set{0};   // one bit per device
-    int dev = 0;
-    TD_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !((attr_set.load() >> dev) & 1ull)) {
-        TD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-        if (dev < 64) attr_set.fetch_or(1ull << dev);
-    }
+    constexpr auto kern = tc_gemm_kernel<MAXC, TF32, NPROD, SWAP, KBYTES>;
+    TD_TRY(allow_smem<kern>(SMEM_MAX));
     const int drain = (op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD)) * (128 / KBYTES);   // in stages
     const dim3 grid((unsigned)std::min<long long>(tiles, sms));
     const unsigned sync_ns = tile_sync_budget_ns();
