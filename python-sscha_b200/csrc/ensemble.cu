@@ -756,13 +756,18 @@ static int freq_ab_drain() {
     return env ? std::max(0, atoi(env)) : 4;
 }
 
-// TDSCHA_FREQ_FUSED_CD=1 forms the thin [c|d] contraction of the split formats inside the weights
-// kernel instead of a grouped contraction plus a separate weights kernel (read at every call).  Off
-// by default: on the 4x4x4 benchmark system the fused kernel takes 6.7 ms per 16-vector step against
-// 2.1 + 3.1 ms for the two launches (same results).
-static bool fused_cd_enabled() {
+// The weights are formed in the epilogue of the [a|b] contraction, which takes [c|d] of the tile as one
+// more chunk (tc::gemm_grouped_weights): a, b, c, d never reach memory.  Contraction, [c|d]
+// and weights apart, then together: 16 vectors on 4x4x4 9.3 + 1.3 + 3.2 -> 11.8 ms; 32 on 3x3x3 1.74 + 0.47 +
+// 1.27 -> 3.02 ms; 32 on 2x2x2 64 + 56 + 191 -> 174 us; 5 on 3x3x3 with N odd (tf32x3) 514 + 95 + 916 -> 984 us.  FP64, chunks over resident rows (two row ranges per
+// class) and classes with more mode columns than the epilogue takes keep the separate launches, as does
+// TDSCHA_FREQ_FUSED_CD=0 (read at every call).
+static bool weights_fused(const FreqTables &t, Format fmt, int nprod) {
     const char *env = getenv("TDSCHA_FREQ_FUSED_CD");
-    return env && atoi(env) == 1;
+    if (fmt == FMT_F64 || (env && atoi(env) == 0)) return false;
+    for (int c : t.mcol_cnt)
+        if (!tc::weights_fit(fmt, nprod, c)) return false;
+    return true;
 }
 
 // An averages call whose operands are built and whose workspace holds all of its rows plans nothing: the
@@ -793,7 +798,8 @@ struct FreqWs {
     long long ld1, ldz, ldf, N2pc;
 };
 
-static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_total, Format fmt, bool lo, long long Nc) {
+// fused: the weights come out of the [a|b] contraction, so H and Ch are not stored
+static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_total, Format fmt, bool lo, long long Nc, bool fused) {
     const FreqTables &t = *e->freq;
     FreqWs L{};
     const size_t es = format_bytes(fmt), as = fmt == FMT_F64 ? 8 : 4;
@@ -810,8 +816,8 @@ static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_t
     L.Lab_lo = lo ? take(2 * NR * t.Kq * es) : 0;
     L.Lcd_hi = take(2 * NR * Kmq * es);
     L.Lcd_lo = lo ? take(2 * NR * Kmq * es) : 0;
-    L.H = take(nC * 2 * NR * L.ld1 * as);
-    L.Ch = take(nC * 2 * NR * L.ld1 * as);
+    L.H = fused ? 0 : take(nC * 2 * NR * L.ld1 * as);
+    L.Ch = fused ? 0 : take(nC * 2 * NR * L.ld1 * as);
     L.Cw_hi = take(nC * 2 * NR * L.N2pc * es);
     L.Cw_lo = lo ? take(nC * 2 * NR * L.N2pc * es) : 0;
     L.AB_hi = take(nC * 2 * NR * L.N2pc * es);
@@ -869,6 +875,7 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
     long long Nc = e->N;
     int ncj = 0;
     bool half = false;   // chunks over resident row-major class operands
+    const bool may_fuse = weights_fused(ft, fmt, nprod);
     FreqOps co;
     if (cap != cudaStreamCaptureStatusNone) {
         const AvgPlan &pl = e->plan;
@@ -886,7 +893,7 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
             co = e->fops[fmt];
         }
     } else if (!chunks_forced() && e->fops[fmt].built && (e->fops[fmt].has_lo || !lo) &&
-               e->ws.bytes >= freq_ws_layout(e, nb, (int)round_up(n_cos, Jf), nf_total, fmt, lo, e->N).total) {
+               e->ws.bytes >= freq_ws_layout(e, nb, (int)round_up(n_cos, Jf), nf_total, fmt, lo, e->N, may_fuse).total) {
         // everything in one pass, with the operands and the workspace of earlier calls: nothing to plan
         ncj = (int)round_up(n_cos, Jf);
         co = e->fops[fmt];
@@ -939,7 +946,7 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
         // coset chunk: the largest multiple of Jf whose workspace fits in the budget
         const size_t budget = std::max<size_t>((size_t)2 << 30, (size_t)((free_b + e->ws.bytes) * 0.6));
         ncj = (int)round_up(n_cos, Jf);
-        while (ncj > Jf && freq_ws_layout(e, nb, ncj, nf_total, fmt, lo, Nc).total > budget) ncj -= Jf;
+        while (ncj > Jf && freq_ws_layout(e, nb, ncj, nf_total, fmt, lo, Nc, may_fuse && !half).total > budget) ncj -= Jf;
         const char *env_sym = getenv("TDSCHA_SYM_CHUNK");   // in symmetries; forces a smaller chunk (tuning and tests)
         if (env_sym && atoi(env_sym) > 0) ncj = std::min(ncj, std::max(Jf, atoi(env_sym) / sub / Jf * Jf));
         e->plan.valid = true;
@@ -953,7 +960,8 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
         e->plan.Jc = ncj * sub;
     }
     const bool chunked = Nc < e->N;
-    const FreqWs L = freq_ws_layout(e, nb, ncj, nf_total, fmt, lo, Nc);
+    const bool fused = may_fuse && !half;
+    const FreqWs L = freq_ws_layout(e, nb, ncj, nf_total, fmt, lo, Nc, fused);
     if (cap != cudaStreamCaptureStatusNone)
         TD_CHECK(e->ws.bytes >= L.total, TDSCHA_EINVAL, "workspace changed since the plan");
     else
@@ -977,8 +985,6 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
     int n_classes = 0;
     for (int m = 1; m <= SYM_MT_MAX; ++m) n_classes += e->pairs.count[m] > 0 ? 1 : 0;
     const long long Kmq1 = std::max(ft.Kmq, 1);
-    bool fused_cd = !f64 && ft.Kmq > 0 && fused_cd_enabled();
-    for (int u : ft.mcol_used) fused_cd = fused_cd && u <= 64;
     for (int p0 = 0; p0 < n_cos; p0 += ncj) {
         const int nc = std::min(ncj, n_cos - p0);
         const int NR = nb * nc;
@@ -1036,21 +1042,24 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
                         gcd.push_back({Mg, (int)N2c, ft.mcol_cnt[g], 0, ft.mcol_off[g], 0, ft.mcol_off[g], hrow * L.ld1});
                     }
                     gf.push_back({Mg, ft.mcol_cnt[g], (int)N2pc, (int)hrow, 0, ft.mcol_off[g], 0, (long long)ft.mcol_off[g]});
-                } else if (!fused_cd) {
+                } else if (!fused) {
                     TD_CUDA(cudaMemsetAsync(static_cast<uint8_t *>(Ch) + hrow * L.ld1 * as, 0, (size_t)2 * NR * L.ld1 * as, st));
                 }
             }
-            {
+            if (fused) {
                 StageScope sc(e, ST_GEMM_AB, st);
-                TD_TRY(gemm_groups(e, fmt, nprod, Lab_hi, Lab_lo, 2LL * NR, ft.Kq, co.V_hi, co.V_lo, brows, ft.Kq, gab, H, L.ld1, false,
-                                   st, freq_ab_drain()));
-            }
-            if (fused_cd) {
-                // [c|d] formed inside the weights kernel (the class's few mode columns)
-                StageScope sc(e, ST_WEIGHTS, st);
-                TD_TRY(freq_weights_cd(ft, (const float *)H, L.ld1, Lcd_hi, Lcd_lo, co.XG_hi, co.XG_lo, e->rho + c0, Ncur, NR, N2pc,
-                                       apply_d4, fmt, Cw_hi, Cw_lo, AB_hi, AB_lo, st));
+                tc::GemmOperands op{fmt, nprod, Lab_hi, Lab_lo, ft.Kq, co.V_hi, co.V_lo, ft.Kq};
+                op.drain_kb = freq_ab_drain();
+                tc::WeightsOut wo{Lcd_hi, Lcd_lo, co.XG_hi, co.XG_lo, ft.Kmq, ft.mcol_cnt, ft.mcol_off, e->rho + c0, (int)Ncur,
+                                  (int)N2pc, apply_d4, Cw_hi, Cw_lo, AB_hi, AB_lo};
+                for (int g = 0; g < nC; ++g) gab[g].d_off = (long long)g * 2 * NR;   // first row of the weights
+                TD_TRY(tc::gemm_grouped_weights(op, 2LL * NR, ft.Kq, brows, ft.Kq, gab.data(), (int)gab.size(), wo, st, e->d_err));
             } else {
+                {
+                    StageScope sc(e, ST_GEMM_AB, st);
+                    TD_TRY(gemm_groups(e, fmt, nprod, Lab_hi, Lab_lo, 2LL * NR, ft.Kq, co.V_hi, co.V_lo, brows, ft.Kq, gab, H, L.ld1,
+                                       false, st, freq_ab_drain()));
+                }
                 {
                     StageScope sc(e, ST_GEMM_CD, st);
                     TD_TRY(gemm_groups(e, fmt, nprod, Lcd_hi, Lcd_lo, 2LL * NR, Kmq1, co.XG_hi, co.XG_lo, brows, Kmq1, gcd, Ch, L.ld1,

@@ -186,7 +186,6 @@ int build_freq_layout(int n, const std::vector<int> &dim, const std::vector<int>
         int mcnt = 0;
         for (int k : mby_cls[g]) { mcomps[k].col = kmq + mcnt; mcnt += mcomps[k].qb >= 0 ? 2 : 1; }
         out.mcol_cnt.push_back(mcnt ? (int)round_up(mcnt, 64) : 0);
-        out.mcol_used.push_back(mcnt);
         kmq += out.mcol_cnt.back();
         (void)id;
     }
@@ -746,98 +745,6 @@ __global__ void __launch_bounds__(256) freq_weights_kernel(const AccT *__restric
     }
 }
 
-template <Format FMT>
-__device__ __forceinline__ float split_value(const void *hi, const void *lo, long long idx) {
-    if constexpr (FMT == FMT_BF16) {
-        float v = bf16_bits_to_float(static_cast<const uint16_t *>(hi)[idx]);
-        if (lo) v += bf16_bits_to_float(static_cast<const uint16_t *>(lo)[idx]);
-        return v;
-    } else {
-        float v = static_cast<const float *>(hi)[idx];
-        if (lo) v += static_cast<const float *>(lo)[idx];
-        return v;
-    }
-}
-
-// One CTA per (32 rows of one class, 128 configurations): the class's mode components of the
-// configurations (x and g) and of the rows' left operands in shared memory (fp32, padded to 65
-// columns), then per (row, configuration) the dot products c, d and the weights.
-template <Format FMT>
-__global__ void __launch_bounds__(256) weights_cd_kernel(const float *__restrict__ H, long long ld, const void *Lcd_hi,
-                                                         const void *Lcd_lo, const void *XG_hi, const void *XG_lo, int Kmq,
-                                                         const double *__restrict__ rho, long long Nc, int NR, int tiles_per_class,
-                                                         const int *__restrict__ cls_real, const int *__restrict__ mcol_off,
-                                                         const int *__restrict__ mcol_used, long long N2pc, int d4, void *Cw_hi,
-                                                         void *Cw_lo, void *AB_hi, void *AB_lo) {
-    extern __shared__ __align__(16) float wsm[];
-    float *Xs = wsm;                   // [128][65]
-    float *Gs = Xs + 128 * 65;         // [128][65]
-    float *Ls = Gs + 128 * 65;         // [32][65]
-    const int g = blockIdx.y;
-    const int Kc = mcol_used[g], moff = mcol_off[g];
-    const bool real_cls = cls_real[g] != 0;
-    const int rows_cls = real_cls ? NR : 2 * NR;
-    const long long i0 = (long long)blockIdx.x * 128;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < 128 * 64; e += 256) {
-        const int ii = e >> 6, cc = e & 63;
-        const long long i = i0 + ii;
-        float xv = 0.f, gv = 0.f;
-        if (cc < Kc && i < Nc) {
-            xv = split_value<FMT>(XG_hi, XG_lo, i * Kmq + moff + cc);
-            gv = split_value<FMT>(XG_hi, XG_lo, (Nc + i) * Kmq + moff + cc);
-        }
-        Xs[ii * 65 + cc] = xv;
-        Gs[ii * 65 + cc] = gv;
-    }
-    const int warp = tid >> 5, lane = tid & 31;
-    const float k4 = d4 ? 1.f : 0.f;
-    // the configuration slice stays in shared memory while the CTA walks every row tile of the class
-    for (int tb = 0; tb * 32 < rows_cls; ++tb) {
-    __syncthreads();
-    for (int e = tid; e < 32 * 64; e += 256) {
-        const int rr = e >> 6, cc = e & 63;
-        const int lr = tb * 32 + rr;   // row inside the class: comp * NR + j
-        float v = 0.f;
-        if (cc < Kc && lr < rows_cls) v = split_value<FMT>(Lcd_hi, Lcd_lo, (long long)lr * Kmq + moff + cc);
-        Ls[rr * 65 + cc] = v;
-    }
-    __syncthreads();
-    for (int rr = warp; rr < 32; rr += 8) {
-        const int lr = tb * 32 + rr;
-        if (lr >= rows_cls) break;
-        const long long r = (long long)g * 2 * NR + lr;
-        const float *h = H + r * ld;
-        const float *l = Ls + rr * 65;
-        for (int q = 0; q < 4; ++q) {
-            const int ii = lane + 32 * q;
-            const long long i = i0 + ii;
-            if (i >= Nc) break;
-            const float *xs = Xs + ii * 65, *gs = Gs + ii * 65;
-            float c = 0.f, d = 0.f;
-            for (int cc = 0; cc < Kc; ++cc) {
-                c = fmaf(l[cc], xs[cc], c);
-                d = fmaf(l[cc], gs[cc], d);
-            }
-            const float a = h[i], b = h[Nc + i];
-            const float rh = (float)rho[i];
-            const float gam = rh * (-c * (1.f / 3.f) + k4 * a * 0.125f);
-            const float hdel = 0.5f * rh * (-d * (1.f / 3.f) + k4 * b * 0.25f);
-            const long long o = r * N2pc;
-            store_split(FMT, Cw_hi, Cw_lo, o + i, (double)hdel);
-            store_split(FMT, Cw_hi, Cw_lo, o + Nc + i, (double)gam);
-            store_split(FMT, AB_hi, AB_lo, o + i, (double)(-rh * a * (1.f / 6.f)));
-            store_split(FMT, AB_hi, AB_lo, o + Nc + i, (double)(-rh * b * (1.f / 3.f)));
-        }
-        if (blockIdx.x == 0)
-            for (long long k = 2 * Nc + lane; k < N2pc; k += 32) {
-                store_split(FMT, Cw_hi, Cw_lo, r * N2pc + k, 0.0);
-                store_split(FMT, AB_hi, AB_lo, r * N2pc + k, 0.0);
-            }
-    }
-    }
-}
-
 }  // namespace
 
 template <typename AccT>
@@ -858,30 +765,6 @@ int freq_weights(const FreqTables &t, const AccT *H, const AccT *Ch, long long l
     return 0;
 }
 
-int freq_weights_cd(const FreqTables &t, const float *H, long long ld, const void *Lcd_hi, const void *Lcd_lo, const void *XG_hi,
-                    const void *XG_lo, const double *rho, long long Nc, int NR, long long N2pc, int d4, Format fmt, void *Cw_hi,
-                    void *Cw_lo, void *AB_hi, void *AB_lo, cudaStream_t st) {
-    TD_CHECK(fmt == FMT_BF16 || fmt == FMT_TF32, TDSCHA_EINVAL, "fused weights need a split format");
-    TD_CHECK(t.Kmq > 0, TDSCHA_EINVAL, "fused weights need mode columns");
-    const int tiles_per_class = ceil_div(2 * NR, 32);
-    const long long gy = t.n_class;
-    const size_t smem = (size_t)(2 * 128 + 32) * 65 * sizeof(float);
-    const dim3 grid((unsigned)ceil_div(Nc, 128), (unsigned)gy);
-    if (fmt == FMT_BF16) {
-        TD_CUDA(cudaFuncSetAttribute(weights_cd_kernel<FMT_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        weights_cd_kernel<FMT_BF16><<<grid, 256, smem, st>>>(H, ld, Lcd_hi, Lcd_lo, XG_hi, XG_lo, t.Kmq, rho, Nc, NR, tiles_per_class,
-                                                             t.d_cls_real, t.d_mcol_off, t.d_mcol_used, N2pc, d4, Cw_hi, Cw_lo,
-                                                             AB_hi, AB_lo);
-    } else {
-        TD_CUDA(cudaFuncSetAttribute(weights_cd_kernel<FMT_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        weights_cd_kernel<FMT_TF32><<<grid, 256, smem, st>>>(H, ld, Lcd_hi, Lcd_lo, XG_hi, XG_lo, t.Kmq, rho, Nc, NR, tiles_per_class,
-                                                             t.d_cls_real, t.d_mcol_off, t.d_mcol_used, N2pc, d4, Cw_hi, Cw_lo,
-                                                             AB_hi, AB_lo);
-    }
-    TD_CUDA(cudaGetLastError());
-    return 0;
-}
-
 template int freq_weights<float>(const FreqTables &, const float *, const float *, long long, const double *, long long, int,
                                  long long, int, Format, void *, void *, void *, void *, cudaStream_t);
 template int freq_weights<double>(const FreqTables &, const double *, const double *, long long, const double *, long long,
@@ -898,7 +781,6 @@ int freq_tables_create(const FreqLayout &L, FreqTables **out) {
     t->pcol_cnt = L.pcol_cnt;
     t->mcol_off = L.mcol_off;
     t->mcol_cnt = L.mcol_cnt;
-    t->mcol_used = L.mcol_used;
     t->flops_ratio = L.flops_ratio;
     size_t acc = 0;
     int rc = 0;
@@ -912,8 +794,7 @@ int freq_tables_create(const FreqLayout &L, FreqTables **out) {
         (rc = upload(L.mc_mode, &t->mc_mode, &acc)) || (rc = upload(L.mc_partner, &t->mc_partner, &acc)) ||
         (rc = upload(L.mode_col, &t->mode_col, &acc)) || (rc = upload(L.mc_sign, &t->mc_sign, &acc)) ||
         (rc = upload(L.mc_re, &t->mc_re, &acc)) || (rc = upload(L.mc_im, &t->mc_im, &acc)) ||
-        (rc = upload(L.mc_zc, &t->mc_zc, &acc)) || (rc = upload(L.cls_real, &t->d_cls_real, &acc)) ||
-        (rc = upload(L.mcol_off, &t->d_mcol_off, &acc)) || (rc = upload(L.mcol_used, &t->d_mcol_used, &acc))) {
+        (rc = upload(L.mc_zc, &t->mc_zc, &acc)) || (rc = upload(L.cls_real, &t->d_cls_real, &acc))) {
         freq_tables_destroy(t);
         return rc;
     }
@@ -926,7 +807,7 @@ void freq_tables_destroy(FreqTables *t) {
     if (!t) return;
     void *ps[] = {t->pc_mu0, t->pc_nu0, t->pc_mu1, t->pc_nu1, t->pc_partner, t->pc_c0, t->pc_c1, t->pc_re, t->pc_im, t->pc_zc,
                   t->pp_col0, t->pp_col1, t->pp_c0, t->pp_c1, t->mc_mode, t->mc_partner, t->mode_col, t->mc_sign, t->mc_re,
-                  t->mc_im, t->mc_zc, t->d_cls_real, t->d_mcol_off, t->d_mcol_used};
+                  t->mc_im, t->mc_zc, t->d_cls_real};
     for (void *p : ps)
         if (p) cudaFree(p);
     delete t;

@@ -37,7 +37,6 @@ struct FreqLayout {
     std::vector<int> cls_real;                        // class is a real character
     std::vector<int> pcol_off, pcol_cnt;              // pair columns of each class (padded)
     std::vector<int> mcol_off, mcol_cnt;              // mode columns of each class (padded; 0 when none)
-    std::vector<int> mcol_used;                       // the class's mode columns before padding
     // per pair column: own value = c0 M[mu0, nu0] + c1 M[mu1, nu1] of a symmetric matrix M
     std::vector<int> pc_mu0, pc_nu0, pc_mu1, pc_nu1;
     std::vector<double> pc_c0, pc_c1;
@@ -61,8 +60,7 @@ int build_freq_layout(int n, const std::vector<int> &dim, const std::vector<int>
 // Device copy of the layout tables.
 struct FreqTables {
     int n_class = 0, Kq = 0, Kmq = 0;
-    std::vector<int> cls_real, pcol_off, pcol_cnt, mcol_off, mcol_cnt, mcol_used;
-    int *d_mcol_off = nullptr, *d_mcol_used = nullptr;   // per class (device)
+    std::vector<int> cls_real, pcol_off, pcol_cnt, mcol_off, mcol_cnt;
     int *pc_mu0 = nullptr, *pc_nu0 = nullptr, *pc_mu1 = nullptr, *pc_nu1 = nullptr, *pc_partner = nullptr;
     double *pc_c0 = nullptr, *pc_c1 = nullptr, *pc_re = nullptr, *pc_im = nullptr, *pc_zc = nullptr;
     int *pp_col0 = nullptr, *pp_col1 = nullptr;
@@ -151,14 +149,6 @@ int freq_vjp_coef(const FreqTables &t, int sub, const AccT *H, const AccT *Ch, c
 template <typename T>
 int freq_vjp_reconstruct(const FreqTables &t, int N, int n, long long P, const T *VbarQ, const T *GQ, const T *YQ, T *Vbar,
                          long long ldv, T *gbar, T *ypart, long long ldg, cudaStream_t st);
-
-// The weights with the thin [c|d] contraction folded in (split formats): c and d of row r and
-// configuration i are the dot products of the row's left operand Lcd (2NR x Kmq, hi + lo) with the
-// configuration's mode components XGq (2Nc x Kmq, hi + lo) over the row's class columns, formed in
-// fp32 next to [a|b] (H) instead of being stored by a contraction and read back.
-int freq_weights_cd(const FreqTables &t, const float *H, long long ld, const void *Lcd_hi, const void *Lcd_lo, const void *XG_hi,
-                    const void *XG_lo, const double *rho, long long Nc, int NR, long long N2pc, int d4, Format fmt, void *Cw_hi,
-                    void *Cw_lo, void *AB_hi, void *AB_lo, cudaStream_t st);
 
 // Back from the character basis: Zs (NR x ldz, packed c_p N~) from O (2 NR x Kq), Fs (NR x ldf)
 // from OF (2 NR x Kmq).

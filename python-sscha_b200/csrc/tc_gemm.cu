@@ -29,6 +29,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -190,6 +191,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Sub-problems of one launch (a single contraction is one group).  Each 128-row tile of the P operand
@@ -198,6 +205,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 constexpr int MAX_GROUPS = 64;
 struct DevGroup {
     int np, nq, K, p_row, p_k, q_row, q_k, tile0, num_p, num_q, tn;
+    int kw, pw_k, qw_k;        // weights epilogue: K and columns of the [c|d] operands
     long long d_off;
 };
 struct GroupTable {
@@ -235,6 +243,7 @@ constexpr int EPI_BUF_FLOATS = 32 * 32;            // one epilogue warp's 32 x 3
 constexpr int SMEM_MAX = 227 * 1024;
 constexpr int SMEM_FIXED = 1024 /*align*/ + 512 /*barriers*/;
 constexpr int EPI_STAGING = EPI_WARPS * EPI_BUF_FLOATS * 4;
+constexpr int epi_staging(bool swap, bool weights) { return swap ? (weights ? 2 * EPI_STAGING : 0) : EPI_STAGING; }
 constexpr uint32_t TMEM_COLS = 512;                // two accumulator buffers of up to 256 columns
 
 template <bool TF32, int KBYTES>
@@ -242,6 +251,198 @@ struct KBlock {
     static constexpr int ELEMS = KBYTES / (TF32 ? 4 : 2);   // K per stage
     static constexpr int UMMA_K = TF32 ? 8 : 16;   // K per instruction (32 bytes)
 };
+
+// What happens to a tile's sums.  EpiArgs<false>: stored to D.  EpiArgs<true>: the averages' weights.  The
+// tile holds a (columns k < Nc) and b (k >= Nc) of its rows; one or two more chunks of the same tile
+// over the rows' and configurations' mode components give c and d, and the stored values are
+//   k < Nc:   Cw[Nc + k] = rho_k (-c/3 + d4 a/8),                AB[k] = -rho_k a/6
+//   k >= Nc:  Cw[k - Nc] = rho_(k-Nc) (-d/3 + d4 b/4) / 2,       AB[k] = -rho_(k-Nc) b/3
+// split into hi / lo, zero from column 2Nc to N2pc.
+template <bool WEIGHTS>
+struct EpiArgs {
+    int unused;
+};
+template <>
+struct EpiArgs<true> {
+    CUtensorMap p_hi, p_lo, q_hi, q_lo;   // operands of [c|d]
+    const double *rho;
+    int Nc, N2pc, d4;
+    int f64;                              // FP64 arithmetic (Nc not a multiple of 4), else fp32
+    int drain_w;                          // stages per chunk of [c|d]
+    void *cw_hi, *cw_lo, *ab_hi, *ab_lo;  // rows of N2pc columns; the group's d_off is its first row
+};
+
+// Correctly rounded x / D for D = 3 or 6 with R = 1 / D rounded: a product, its exact remainder and a
+// correction (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990,
+// theorem on quotients from a correctly rounded reciprocal); three FP64 instructions instead of a division.
+template <int D>
+__device__ __forceinline__ double div_const(double x) {
+    constexpr double R = 1.0 / D;
+    const double q = x * R;
+    const double r = __fma_rn(__fma_rn(-(double)D, q, x), R, q);
+    return isfinite(q) ? r : q;
+}
+
+// hi and lo of two weights in the storage format, as bits (bf16: packed into one word each).  Products and
+// differences are rounded one by one.
+template <bool TF32, typename T>
+struct Split2 {
+    uint32_t h0, h1, l0, l1;   // tf32: one word per weight; bf16: h0, l0 hold both
+    __device__ __forceinline__ Split2(T x0, T x1) {
+        if constexpr (TF32) {
+            const float f0 = tf32_round((float)x0), f1 = tf32_round((float)x1);
+            h0 = __float_as_uint(f0);
+            h1 = __float_as_uint(f1);
+            if constexpr (sizeof(T) == 8) {
+                l0 = __float_as_uint(tf32_round((float)(x0 - (double)f0)));
+                l1 = __float_as_uint(tf32_round((float)(x1 - (double)f1)));
+            } else {
+                l0 = __float_as_uint(tf32_round(__fsub_rn(x0, f0)));
+                l1 = __float_as_uint(tf32_round(__fsub_rn(x1, f1)));
+            }
+        } else {
+            h0 = pack((float)x0, (float)x1);
+            const float f0 = __uint_as_float(h0 << 16), f1 = __uint_as_float(h0 & 0xffff0000u);
+            if constexpr (sizeof(T) == 8) l0 = pack((float)(x0 - (double)f0), (float)(x1 - (double)f1));
+            else l0 = pack(__fsub_rn(x0, f0), __fsub_rn(x1, f1));
+            h1 = l1 = 0;
+        }
+    }
+    static __device__ __forceinline__ uint32_t pack(float a, float b) {   // a in the low half
+        uint32_t r;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+        return r;
+    }
+};
+
+// The factors of one configuration column (first: a and c, else b and d) and the weights of one element,
+// v = a or b, w = c or d, in T = float or double arithmetic.
+template <typename T>
+struct WeightCol {
+    T rc, ra, s;   // of Cw; of AB; of v in Cw (0 without d4)
+    bool first;
+    __device__ __forceinline__ WeightCol() {}
+    __device__ __forceinline__ WeightCol(double rho, bool first_, int d4) : first(first_) {
+        if constexpr (sizeof(T) == 8) {
+            rc = first ? rho : 0.5 * rho;
+            ra = -rho;
+            s = d4 ? (first ? 0.125 : 0.25) : 0.0;
+        } else {
+            const float r = (float)rho;
+            rc = first ? r : 0.5f * r;
+            ra = -r;
+            s = d4 ? (first ? 0.125f : 0.25f) : 0.f;
+        }
+    }
+    __device__ __forceinline__ T cw(float v, float w) const {
+        if constexpr (sizeof(T) == 8) return rc * (div_const<3>(-(double)w) + (s != 0.0 ? (double)v * s : 0.0));
+        else return __fmul_rn(rc, __fmaf_rn(v, s, __fmul_rn(-w, 1.f / 3.f)));   // v s is exact: rounded once
+    }
+    __device__ __forceinline__ T ab(float v) const {
+        if constexpr (sizeof(T) == 8) {
+            const double y = ra * (double)v;
+            return first ? div_const<6>(y) : div_const<3>(y);
+        } else {
+            return __fmul_rn(__fmul_rn(ra, v), first ? 1.f / 6.f : 1.f / 3.f);
+        }
+    }
+};
+// One weight, hi and lo, at element `i` of the output arrays
+template <bool TF32, int NPROD>
+__device__ __forceinline__ void store_weight(void *hi, void *lo, long long i, uint32_t h, uint32_t l) {
+    if constexpr (TF32) {
+        static_cast<uint32_t *>(hi)[i] = h;
+        if (NPROD == 3) static_cast<uint32_t *>(lo)[i] = l;
+    } else {
+        static_cast<uint16_t *>(hi)[i] = (uint16_t)h;
+        if (NPROD == 3) static_cast<uint16_t *>(lo)[i] = (uint16_t)l;
+    }
+}
+
+// 32 rows x 16 columns of a tile: v in the first half of the warp's block, w in the second, 16-byte chunks
+// XOR-swizzled (chunk j of row r at j ^ (r / 2 & 3)).
+// fp32 arithmetic (Nc a multiple of 4): lane = (row of 8, chunk of 4 columns, all a or all b), vector stores.
+template <bool TF32, int NPROD>
+__device__ __forceinline__ void weights_block_f32(const EpiArgs<true> &ea, const float *wbuf, long long row0, int rows, int k0, int k_end) {
+    const int lane = threadIdx.x & 31, rsub = lane >> 2, chk = lane & 3;
+    const int k = k0 + 4 * chk, Nc = ea.Nc;
+    if (k >= k_end) return;   // k_end is a multiple of 4 here
+    WeightCol<float> col[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) col[e] = WeightCol<float>(__ldg(ea.rho + (k < Nc ? k + e : k + e - Nc)), k < Nc, ea.d4);
+    using E = typename std::conditional<TF32, float, uint16_t>::type;
+    const long long o = (row0 + rsub) * ea.N2pc, oc = o + (k < Nc ? Nc + k : k - Nc);
+    E *ch = static_cast<E *>(ea.cw_hi) + oc, *cl = static_cast<E *>(ea.cw_lo) + oc;
+    E *ah = static_cast<E *>(ea.ab_hi) + o + k, *al = static_cast<E *>(ea.ab_lo) + o + k;
+#pragma unroll 2
+    for (int i = rsub; i < rows; i += 8) {
+        const int c = i * 16 + 4 * (chk ^ ((i >> 1) & 3));
+        const float4 v = *reinterpret_cast<const float4 *>(wbuf + c), w = *reinterpret_cast<const float4 *>(wbuf + 512 + c);
+        const Split2<TF32, float> c0(col[0].cw(v.x, w.x), col[1].cw(v.y, w.y)), c1(col[2].cw(v.z, w.z), col[3].cw(v.w, w.w));
+        const Split2<TF32, float> a0(col[0].ab(v.x), col[1].ab(v.y)), a1(col[2].ab(v.z), col[3].ab(v.w));
+        const long long d = (long long)(i - rsub) * ea.N2pc;
+        if constexpr (TF32) {
+            *reinterpret_cast<uint4 *>(ch + d) = make_uint4(c0.h0, c0.h1, c1.h0, c1.h1);
+            *reinterpret_cast<uint4 *>(ah + d) = make_uint4(a0.h0, a0.h1, a1.h0, a1.h1);
+            if (NPROD == 3) {
+                *reinterpret_cast<uint4 *>(cl + d) = make_uint4(c0.l0, c0.l1, c1.l0, c1.l1);
+                *reinterpret_cast<uint4 *>(al + d) = make_uint4(a0.l0, a0.l1, a1.l0, a1.l1);
+            }
+        } else {
+            *reinterpret_cast<uint2 *>(ch + d) = make_uint2(c0.h0, c1.h0);
+            *reinterpret_cast<uint2 *>(ah + d) = make_uint2(a0.h0, a1.h0);
+            if (NPROD == 3) {
+                *reinterpret_cast<uint2 *>(cl + d) = make_uint2(c0.l0, c1.l0);
+                *reinterpret_cast<uint2 *>(al + d) = make_uint2(a0.l0, a1.l0);
+            }
+        }
+    }
+}
+// FP64 arithmetic (any Nc): lane = (row of 2, column), so that 16 lanes store 16 neighbouring elements.
+template <bool TF32, int NPROD>
+__device__ __forceinline__ void weights_block_f64(const EpiArgs<true> &ea, const float *wbuf, long long row0, int rows, int k0, int k_end) {
+    const int lane = threadIdx.x & 31, rsub = lane >> 4, c = lane & 15;
+    const int k = k0 + c, Nc = ea.Nc;
+    if (k >= k_end) return;
+    const WeightCol<double> col(__ldg(ea.rho + (k < Nc ? k : k - Nc)), k < Nc, ea.d4);
+    const int kc = k < Nc ? Nc + k : k - Nc;
+#pragma unroll 1
+    for (int i = rsub; i < rows; i += 4) {   // two rows of the lane at a time
+        const int i1 = min(i + 2, rows - 1);
+        const int c0 = i * 16 + 4 * ((c >> 2) ^ ((i >> 1) & 3)) + (c & 3), c1 = i1 * 16 + 4 * ((c >> 2) ^ ((i1 >> 1) & 3)) + (c & 3);
+        const Split2<TF32, double> x(col.cw(wbuf[c0], wbuf[512 + c0]), col.cw(wbuf[c1], wbuf[512 + c1]));
+        const Split2<TF32, double> y(col.ab(wbuf[c0]), col.ab(wbuf[c1]));
+        const long long o = (row0 + i) * ea.N2pc, o1 = o + 2LL * ea.N2pc;
+        store_weight<TF32, NPROD>(ea.cw_hi, ea.cw_lo, o + kc, x.h0, x.l0);
+        store_weight<TF32, NPROD>(ea.ab_hi, ea.ab_lo, o + k, y.h0, y.l0);
+        if (i + 2 < rows) {
+            store_weight<TF32, NPROD>(ea.cw_hi, ea.cw_lo, o1 + kc, TF32 ? x.h1 : x.h0 >> 16, TF32 ? x.l1 : x.l0 >> 16);
+            store_weight<TF32, NPROD>(ea.ab_hi, ea.ab_lo, o1 + k, TF32 ? y.h1 : y.h0 >> 16, TF32 ? y.l1 : y.l0 >> 16);
+        }
+    }
+}
+
+// `rows` rows of a swapped tile, this lane's configuration k: v (row, lane) in the first of the warp's two
+// blocks, w in the second.
+template <bool TF32, int NPROD, typename T>
+__device__ __forceinline__ void weights_rows_of(const EpiArgs<true> &ea, const float *wbuf, long long row0, int rows, int k, double rho) {
+    const int lane = threadIdx.x & 31;
+    const WeightCol<T> col(rho, k < ea.Nc, ea.d4);
+    const int kc = k < ea.Nc ? ea.Nc + k : k - ea.Nc;
+#pragma unroll(sizeof(T) == 8 ? 1 : 2)
+    for (int i = 0; i < rows; i += 2) {   // row i + 1 is in the block even where it is not stored
+        const float v0 = wbuf[i * 32 + lane], v1 = wbuf[i * 32 + 32 + lane];
+        const float w0 = wbuf[1024 + i * 32 + lane], w1 = wbuf[1024 + i * 32 + 32 + lane];
+        const Split2<TF32, T> x(col.cw(v0, w0), col.cw(v1, w1)), y(col.ab(v0), col.ab(v1));
+        const long long o = (row0 + i) * ea.N2pc, o1 = o + ea.N2pc;
+        store_weight<TF32, NPROD>(ea.cw_hi, ea.cw_lo, o + kc, x.h0, x.l0);
+        store_weight<TF32, NPROD>(ea.ab_hi, ea.ab_lo, o + k, y.h0, y.l0);
+        if (i + 1 < rows) {
+            store_weight<TF32, NPROD>(ea.cw_hi, ea.cw_lo, o1 + kc, TF32 ? x.h1 : x.h0 >> 16, TF32 ? x.l1 : x.l0 >> 16);
+            store_weight<TF32, NPROD>(ea.ab_hi, ea.ab_lo, o1 + k, TF32 ? y.h1 : y.h0 >> 16, TF32 ? y.l1 : y.l0 >> 16);
+        }
+    }
+}
 
 // Persistent: CTA c processes tiles c, c + gridDim.x, ...  Each tile's K loop is split into chunks
 // of `drain` k-blocks; a chunk accumulates from zero in one of two TMEM buffers (the MMA warp moves on
@@ -261,12 +462,13 @@ struct KBlock {
 //         MMA's N side, which steps by 16, instead of padding them to 128-row tiles.
 // The three split products of a k-step are issued hi.hi, A_hi.B_lo, A_lo.B_hi in both orientations and
 // for every width, so each output is the same sum in the same order whatever tile computes it.
-template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES>
+template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES, bool WEIGHTS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant__ CUtensorMap tmP_lo,
                const __grid_constant__ CUtensorMap tmQ_hi, const __grid_constant__ CUtensorMap tmQ_lo,
                const __grid_constant__ GroupTable gt, int drain, int group_p, float *__restrict__ D, long long ldd, unsigned *err,
-               unsigned *tile_sync, unsigned sync_ns, int accumulate, unsigned long long wait_ns, int stall) {
+               unsigned *tile_sync, unsigned sync_ns, int accumulate, unsigned long long wait_ns, int stall,
+               const __grid_constant__ EpiArgs<WEIGHTS> ea) {
     using KB = KBlock<TF32, KBYTES>;
     constexpr int EPI_COLS = MAXC / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -313,7 +515,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant
     if ((warp == 0 || warp == 10 || (warp == 11 && NPROD == 3)) && !stall) {
         // ---------------- TMA producers: P (hi and lo), Q hi, Q lo ----------------
         const uint32_t leader = elect_one();
-        const CUtensorMap *map = warp == 0 ? &tmP_hi : (warp == 10 ? &tmQ_hi : &tmQ_lo);
+        const CUtensorMap *map0 = warp == 0 ? &tmP_hi : (warp == 10 ? &tmQ_hi : &tmQ_lo), *map = map0;
         if (leader) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
         const uint32_t dst0 = smem0 + (warp == 0 ? 0 : gt.q_off + (warp == 10 ? 0 : gt.q_bytes));
         int s = 0;
@@ -343,14 +545,25 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant
                 nbox = (min(G.tn, G.nq - qb * G.tn) + box - 1) / box;
             }
             const uint32_t tx = (uint32_t)((warp == 0 && NPROD == 3 ? 2 : nbox) * box * KBYTES);
-            for (int kb = 0; kb < num_kb; ++kb, kc += KB::ELEMS) {
+            int kb_all = num_kb;
+            if constexpr (WEIGHTS) kb_all += G.kw / KB::ELEMS;
+            const CUtensorMap *map_lo = &tmP_lo;
+            map = map0;
+            for (int kb = 0; kb < kb_all; ++kb, kc += KB::ELEMS) {
+                if constexpr (WEIGHTS) {
+                    if (kb == num_kb) {   // the [c|d] chunks of the tile
+                        map = warp == 0 ? &ea.p_hi : (warp == 10 ? &ea.q_hi : &ea.q_lo);
+                        map_lo = &ea.p_lo;
+                        kc = warp == 0 ? G.pw_k : G.qw_k;
+                    }
+                }
                 if (!mbar_wait(bar0 + 8 * (MAX_STAGES + s), ph, abort_flag, wait_ns)) { ok = false; break; }
                 if (leader) {
                     const uint32_t dst = dst0 + s * stage_bytes, full = bar0 + 8 * s;
                     mbar_expect_tx(full, tx);
                     tma_load_2d(dst, map, kc, row, full);
                     if (warp == 0) {
-                        if constexpr (NPROD == 3) tma_load_2d(dst + (gt.q_off >> 1), &tmP_lo, kc, row, full);
+                        if constexpr (NPROD == 3) tma_load_2d(dst + (gt.q_off >> 1), map_lo, kc, row, full);
                     } else {
                         for (int i = 1; i < nbox; ++i) tma_load_2d(dst + i * box * KBYTES, map, kc, row + i * box, full);
                     }
@@ -376,14 +589,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant
             const int ncol = (min(G.tn, G.nq - qb * G.tn) + 15) & ~15;
             const uint32_t idesc = make_idesc(TF32, gt.p_rows, ncol);
             const int num_kb = G.K / KB::ELEMS;
-            for (int k0 = 0; k0 < num_kb && ok; k0 += drain, ++ch) {
+            int kb_all = num_kb;
+            if constexpr (WEIGHTS) kb_all += G.kw / KB::ELEMS;
+            for (int k0 = 0, k1; k0 < kb_all && ok; k0 = k1, ++ch) {
+                k1 = min(num_kb, k0 + drain);
+                if constexpr (WEIGHTS) {
+                    if (k0 >= num_kb) k1 = min(kb_all, k0 + ea.drain_w);
+                }
                 const uint32_t X = ch & 1u;
                 if (!mbar_wait(smem_u32(&acc_empty[X]), ((ch >> 1) & 1u) ^ 1u, abort_flag, wait_ns)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t dtm = tmem_base + X * 256u;
-                const int kb_end = min(num_kb, k0 + drain);
                 uint32_t acc = 0;
-                for (int kb = k0; kb < kb_end; ++kb) {
+                for (int kb = k0; kb < k1; ++kb) {
                     if (!mbar_wait(bar0 + 8 * s, ph, abort_flag, wait_ns)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t d = desc0 + (uint32_t)s * stage_d;
@@ -449,7 +667,106 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmP_hi, const __grid_constant
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[X])) : "memory");
             }
             if (!ok) break;
-            if constexpr (SWAP) {
+            if constexpr (WEIGHTS) {
+                // [c|d]: none, one or two chunks, summed in fp32 as the others
+                const int nw = (G.kw / KB::ELEMS + ea.drain_w - 1) / ea.drain_w;
+                for (int x = 0; x < nw && ok; ++x)
+                    ok = mbar_wait(smem_u32(&acc_full[(ch + x) & 1u]), ((ch + x) >> 1) & 1u, abort_flag, wait_ns);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c_lo;
+                const uint32_t t0 = tq + (ch & 1u) * 256u, t1 = tq + ((ch + 1) & 1u) * 256u;
+                const int p0 = pb * gt.p_rows + q * rq, q0 = qb * G.tn + c_lo;
+                float *wbuf = epi_buf + ew * EPI_BUF_FLOATS * (SWAP ? 2 : 1);
+                auto release = [&]() {   // after the last read of the buffers
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    for (int x = 0; x < nw; ++x)
+                        if (lane == 0)
+                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[(ch + x) & 1u])) : "memory");
+                };
+                auto load_w = [&](int col, float (&w)[16]) {   // c or d of 16 columns, summed over its chunks
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) w[i] = 0.f;
+                    if (nw > 0) {
+                        uint32_t r[16];
+                        tmem_ld16(t0 + (uint32_t)col, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) w[i] += __uint_as_float(r[i]);
+                        if (nw > 1) {
+                            tmem_ld16(t1 + (uint32_t)col, r);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) w[i] += __uint_as_float(r[i]);
+                        }
+                    }
+                };
+                // The sums leave the registers through the warp's 4 KB block and are worked on in small
+                // loops: unrolled over all 128 registers the arithmetic overran the instruction cache
+                // (about 120 us a tile instead of 16).
+                if constexpr (SWAP) {
+                    // lane = configuration, block row = output row: a store of the warp is a row's 64 or 128
+                    // contiguous bytes
+                    const int k = p0 + lane;
+                    const bool mine = lane < rq && k < G.np;
+                    const double rho = mine ? __ldg(ea.rho + (k < ea.Nc ? k : k - ea.Nc)) : 0.0;
+#pragma unroll
+                    for (int sub = 0; sub < EPI_COLS / 32; ++sub) {
+                        if (sub >= nsub) break;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) wbuf[i * 32 + lane] = acc[sub * 32 + i];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            float w[16];
+                            load_w(sub * 32 + j * 16, w);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) wbuf[1024 + (j * 16 + i) * 32 + lane] = w[i];
+                        }
+                        if (sub + 1 == nsub) release();
+                        const int rows = min(32, width - c_lo - sub * 32);
+                        if (mine) {   // every lane reads only what it wrote
+                            if (ea.f64) weights_rows_of<TF32, NPROD, double>(ea, wbuf, G.d_off + q0 + sub * 32, rows, k, rho);
+                            else weights_rows_of<TF32, NPROD, float>(ea, wbuf, G.d_off + q0 + sub * 32, rows, k, rho);
+                        }
+                        __syncwarp();
+                    }
+                } else {
+                    // lane = row, register = configuration column: 16 columns at a time, transposed in the block
+                    // so that a store covers 32 (bf16) or 64 contiguous bytes of each of 8 rows
+#pragma unroll
+                    for (int p = 0; p < EPI_COLS / 16; ++p) {
+                        if (p * 16 >= min(hw, width - c_lo)) break;
+                        float w[16];
+                        load_w(p * 16, w);
+                        if ((p + 1) * 16 >= min(hw, width - c_lo)) release();
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int c = 4 * (j ^ ((lane >> 1) & 3));
+                            *reinterpret_cast<float4 *>(wbuf + lane * 16 + c) =
+                                make_float4(acc[p * 16 + 4 * j], acc[p * 16 + 4 * j + 1], acc[p * 16 + 4 * j + 2], acc[p * 16 + 4 * j + 3]);
+                            *reinterpret_cast<float4 *>(wbuf + 512 + lane * 16 + c) = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                        }
+                        __syncwarp();
+                        if (ea.f64) weights_block_f64<TF32, NPROD>(ea, wbuf, G.d_off + p0, min(rq, G.np - p0), q0 + p * 16, qb * G.tn + width);
+                        else weights_block_f32<TF32, NPROD>(ea, wbuf, G.d_off + p0, min(rq, G.np - p0), q0 + p * 16, qb * G.tn + width);
+                        __syncwarp();   // the block is rewritten by the next 16 columns
+                    }
+                }
+                if (nsub <= 0) release();
+                ch += nw;
+                // zero columns past 2Nc, by the tile that ends there
+                const int rows = SWAP ? width : min(gt.p_rows, G.np - pb * gt.p_rows);
+                const bool last = SWAP ? (pb + 1) * gt.p_rows >= G.np : qb * G.tn + width >= G.nq;
+                if (last)
+                    for (int i = ew; i < rows; i += EPI_WARPS) {
+                        const long long o = (G.d_off + (SWAP ? qb * G.tn : pb * gt.p_rows) + i) * (long long)ea.N2pc;
+                        for (int k = 2 * ea.Nc + lane; k < ea.N2pc; k += 32) {
+                            store_weight<TF32, NPROD>(ea.cw_hi, ea.cw_lo, o + k, 0u, 0u);
+                            store_weight<TF32, NPROD>(ea.ab_hi, ea.ab_lo, o + k, 0u, 0u);
+                        }
+                    }
+            } else if constexpr (SWAP) {
                 // lane = output column (P row), register = output row (Q row): each register is one
                 // coalesced 128-byte store of the warp
                 const int m = pb * gt.p_rows + q * rq + lane;
@@ -705,8 +1022,8 @@ struct Prepared {
     long long tiles = 0;
 };
 
-template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES>
-static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
+template <int MAXC, bool TF32, int NPROD, bool SWAP, int KBYTES, bool WEIGHTS>
+static int prepare_cfg(const GemmOperands &op, const WeightsOut *wo, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
                        long long ldd, cudaStream_t st, unsigned *err, unsigned *counter, int stall, int sms, Prepared *out) {
     CUtensorMap p_hi, p_lo, q_hi, q_lo;
     const int a_box = SWAP ? pl.q_box : pl.p_box, b_box = SWAP ? pl.p_box : pl.q_box;
@@ -729,7 +1046,7 @@ static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, siz
     gt.q_off = NOPS * sh.p_rows * KBYTES;
     gt.q_bytes = pl.q_rows * KBYTES;
     gt.stage_bytes = gt.q_off + NOPS * gt.q_bytes;
-    const int staging = SWAP ? 0 : EPI_STAGING;
+    const int staging = epi_staging(SWAP, WEIGHTS);
     gt.stages = std::min(MAX_STAGES, (SMEM_MAX - SMEM_FIXED - staging) / gt.stage_bytes);
     TD_CHECK(gt.stages >= 2, TDSCHA_EINVAL, "tc::gemm: tile of %d rows does not fit", pl.q_rows);
     const int smem = gt.stages * gt.stage_bytes + SMEM_FIXED + staging;
@@ -745,6 +1062,10 @@ static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, siz
         d.q_row = SWAP ? g.a_row : g.b_row;
         d.q_k = SWAP ? g.a_k : g.b_k;
         d.d_off = g.d_off;
+        if (WEIGHTS) {
+            d.kw = wo->K[i];
+            d.pw_k = d.qw_k = wo->col[i];
+        }
         d.tn = tile_width(d.nq, sh.cap);
         d.num_p = ceil_div(d.np, sh.p_rows);
         d.num_q = ceil_div(d.nq, d.tn);
@@ -753,7 +1074,7 @@ static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, siz
     }
     TD_CHECK(tiles < (1LL << 31), TDSCHA_EINVAL, "tc::gemm: %lld tiles exceed the schedule", tiles);
     gt.total_tiles = (int)tiles;
-    constexpr auto kern = tc_gemm_kernel<MAXC, TF32, NPROD, SWAP, KBYTES>;
+    constexpr auto kern = tc_gemm_kernel<MAXC, TF32, NPROD, SWAP, KBYTES, WEIGHTS>;
     TD_TRY(allow_smem<kern>(SMEM_MAX));
     const int drain = (op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD)) * (128 / KBYTES);   // in stages
     const dim3 grid((unsigned)std::min<long long>(tiles, sms));
@@ -766,32 +1087,53 @@ static int prepare_cfg(const GemmOperands &op, const Problem &pb, size_t g0, siz
     int k_max = 0;
     for (size_t i = g0; i < g1; ++i) k_max = std::max(k_max, pb.groups[i].K);
     unsigned *cnt = (sync_ns > 0 && tiles > grid.x && k_max >= 32768) ? counter : nullptr;
+    EpiArgs<WEIGHTS> ea{};
+    if constexpr (WEIGHTS) {
+        CUtensorMap *wa[2] = {SWAP ? &ea.q_hi : &ea.p_hi, SWAP ? &ea.q_lo : &ea.p_lo}, *wb[2] = {SWAP ? &ea.p_hi : &ea.q_hi, SWAP ? &ea.p_lo : &ea.q_lo};
+        if (wo->ld > 0) {
+            for (int x = 0; x < (NPROD == 3 ? 2 : 1); ++x) {
+                TD_TRY(make_map(wa[x], x ? wo->A_lo : wo->A_hi, TF32, pb.a_rows, wo->ld, wo->ld, a_box, KBYTES));
+                TD_TRY(make_map(wb[x], x ? wo->B_lo : wo->B_hi, TF32, pb.b_rows, wo->ld, wo->ld, b_box, KBYTES));
+            }
+        }
+        ea.rho = wo->rho;
+        ea.Nc = wo->Nc;
+        ea.N2pc = wo->N2pc;
+        ea.d4 = wo->d4;
+        ea.f64 = wo->Nc % 4 != 0;
+        ea.drain_w = default_drain(NPROD) * (128 / KBYTES);
+        ea.cw_hi = wo->cw_hi; ea.cw_lo = wo->cw_lo; ea.ab_hi = wo->ab_hi; ea.ab_lo = wo->ab_lo;
+    }
     out->num_p = pl.max_p;
     out->shape = sh;
     out->tiles = tiles;
     out->launch = [=](int gp) {
         if (cnt) cudaMemsetAsync(cnt, 0, sizeof(unsigned), st);
         kern<<<grid, NUM_THREADS, smem, st>>>(p_hi, p_lo, q_hi, q_lo, gt, drain, gp, D, ldd, err, cnt, sync_ns, accumulate, wait_ns,
-                                              stall);
+                                              stall, ea);
     };
     return 0;
 }
 
 template <bool TF32, int NPROD>
-static int prepare(const GemmOperands &op, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
+static int prepare(const GemmOperands &op, const WeightsOut *wo, const Problem &pb, size_t g0, size_t g1, TileShape sh, const TilePlan &pl, float *D,
                    long long ldd, cudaStream_t st, unsigned *err, unsigned *counter, int stall, int sms, Prepared *out) {
     const int c = sh.cap <= 64 ? 64 : (sh.cap <= 128 ? 128 : 256);
     // half stages where full ones would leave the ring two deep
     constexpr int NOPS = NPROD == 3 ? 2 : 1;
-    const int room = SMEM_MAX - SMEM_FIXED - (sh.swap ? 0 : EPI_STAGING);
+    const int room = SMEM_MAX - SMEM_FIXED - epi_staging(sh.swap, wo != nullptr);
     const bool half = c == 256 && room / (NOPS * 128 * (sh.p_rows + pl.q_rows)) < 3;
-#define TD_PREP(C, SW, KBY) prepare_cfg<C, TF32, NPROD, SW, KBY>(op, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, out)
-    if (sh.swap) {
-        if (half) return TD_PREP(256, true, 64);
-        return c == 64 ? TD_PREP(64, true, 128) : (c == 128 ? TD_PREP(128, true, 128) : TD_PREP(256, true, 128));
+#define TD_PREP(C, SW, KBY, W) prepare_cfg<C, TF32, NPROD, SW, KBY, W>(op, wo, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, out)
+    if (wo) {
+        if (sh.swap) return half ? TD_PREP(256, true, 64, true) : TD_PREP(256, true, 128, true);
+        return half ? TD_PREP(256, false, 64, true) : TD_PREP(256, false, 128, true);
     }
-    if (half) return TD_PREP(256, false, 64);
-    return c == 64 ? TD_PREP(64, false, 128) : (c == 128 ? TD_PREP(128, false, 128) : TD_PREP(256, false, 128));
+    if (sh.swap) {
+        if (half) return TD_PREP(256, true, 64, false);
+        return c == 64 ? TD_PREP(64, true, 128, false) : (c == 128 ? TD_PREP(128, true, 128, false) : TD_PREP(256, true, 128, false));
+    }
+    if (half) return TD_PREP(256, false, 64, false);
+    return c == 64 ? TD_PREP(64, false, 128, false) : (c == 128 ? TD_PREP(128, false, 128, false) : TD_PREP(256, false, 128, false));
 #undef TD_PREP
 }
 
@@ -895,7 +1237,7 @@ static TileShape choose_shape(const Problem &pb, size_t g0, size_t g1, const Tun
 }
 
 template <bool TF32, int NPROD>
-static int launch_tuned(const GemmOperands &op, const Problem &pb, float *D, long long ldd, cudaStream_t st, unsigned *err) {
+static int launch_tuned(const GemmOperands &op, const WeightsOut *wo, const Problem &pb, float *D, long long ldd, cudaStream_t st, unsigned *err) {
     int dev = 0, sms = 148;
     TD_CUDA(cudaGetDevice(&dev));
     TD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -922,7 +1264,7 @@ static int launch_tuned(const GemmOperands &op, const Problem &pb, float *D, lon
         TilePlan pl;
         const TileShape sh = choose_shape(pb, g0, g1, key, KBlock<TF32, 128>::ELEMS, NPROD, drain, sms, stall != 0, &pl);
         Prepared cfg;
-        TD_TRY((prepare<TF32, NPROD>(op, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, &cfg)));
+        TD_TRY((prepare<TF32, NPROD>(op, wo, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, &cfg)));
         int gp = cfg.num_p;
         // trial runs write D, so an accumulating launch only reuses a choice tuned earlier (and a launch
         // being captured into a CUDA graph runs nothing, so it cannot time trials); the abort-path
@@ -938,13 +1280,14 @@ void set_wait_budget_ns(unsigned long long ns) { g_wait_budget_ns.store(ns); }
 unsigned long long wait_budget_ns() { return g_wait_budget_ns.load(); }
 void stall_next_launch() { g_stall_next.store(1); }
 
-static int dispatch(const GemmOperands &op, const Problem &pb, float *D, long long ldd, cudaStream_t st, unsigned *err) {
+static int dispatch(const GemmOperands &op, const WeightsOut *wo, const Problem &pb, float *D, long long ldd, cudaStream_t st,
+                    unsigned *err) {
     if (op.fmt == FMT_TF32) {
-        if (op.nprod == 3) return launch_tuned<true, 3>(op, pb, D, ldd, st, err);
-        return launch_tuned<true, 1>(op, pb, D, ldd, st, err);
+        if (op.nprod == 3) return launch_tuned<true, 3>(op, wo, pb, D, ldd, st, err);
+        return launch_tuned<true, 1>(op, wo, pb, D, ldd, st, err);
     }
-    if (op.nprod == 3) return launch_tuned<false, 3>(op, pb, D, ldd, st, err);
-    return launch_tuned<false, 1>(op, pb, D, ldd, st, err);
+    if (op.nprod == 3) return launch_tuned<false, 3>(op, wo, pb, D, ldd, st, err);
+    return launch_tuned<false, 1>(op, wo, pb, D, ldd, st, err);
 }
 
 int gemm(const GemmOperands &op, int M, int N, int K, float *D, long long ldd, cudaStream_t st, unsigned *err) {
@@ -958,11 +1301,11 @@ int gemm(const GemmOperands &op, int M, int N, int K, float *D, long long ldd, c
              "tc::gemm: leading dimensions lda=%lld ldb=%lld ldd=%lld inconsistent with K=%d N=%d", op.lda, op.ldb, ldd, K, N);
     TD_CHECK(op.A_hi && op.B_hi && D && (op.nprod == 1 || (op.A_lo && op.B_lo)), TDSCHA_EINVAL, "tc::gemm: NULL operand");
     Problem pb{M, K, N, K, {GemmGroup{M, N, K, 0, 0, 0, 0, 0}}};
-    return dispatch(op, pb, D, ldd, st, err);
+    return dispatch(op, nullptr, pb, D, ldd, st, err);
 }
 
-int gemm_grouped(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
-                 const GemmGroup *groups, int n_groups, float *D, long long ldd, cudaStream_t st, unsigned *err) {
+static int check_groups(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
+                        const GemmGroup *groups, int n_groups, long long ldd, Problem *out) {
     TD_CHECK(n_groups > 0 && groups, TDSCHA_EINVAL, "tc::gemm_grouped: no groups");
     const bool tf32 = op.fmt == FMT_TF32;
     TD_CHECK(op.fmt == FMT_TF32 || op.fmt == FMT_BF16, TDSCHA_EINVAL, "tc::gemm_grouped: operand format must be bf16 or tf32");
@@ -972,8 +1315,9 @@ int gemm_grouped(const GemmOperands &op, long long a_rows, long long a_cols, lon
     TD_CHECK(op.lda >= a_cols && op.ldb >= b_cols && op.lda < LD_MAX && op.ldb < LD_MAX && ldd < LD_MAX && a_rows < LD_MAX &&
                  b_rows < LD_MAX && a_cols < LD_MAX && b_cols < LD_MAX,
              TDSCHA_EINVAL, "tc::gemm_grouped: operand extents inconsistent with their leading dimensions");
-    TD_CHECK(op.A_hi && op.B_hi && D && (op.nprod == 1 || (op.A_lo && op.B_lo)), TDSCHA_EINVAL, "tc::gemm_grouped: NULL operand");
-    Problem pb{a_rows, a_cols, b_rows, b_cols, {}};
+    TD_CHECK(op.A_hi && op.B_hi && (op.nprod == 1 || (op.A_lo && op.B_lo)), TDSCHA_EINVAL, "tc::gemm_grouped: NULL operand");
+    Problem &pb = *out;
+    pb = Problem{a_rows, a_cols, b_rows, b_cols, {}};
     for (int i = 0; i < n_groups; ++i) {
         const GemmGroup &g = groups[i];
         TD_CHECK(g.M > 0 && g.N > 0 && g.K > 0 && g.K % kblk == 0 && g.a_k % kblk == 0 && g.b_k % kblk == 0, TDSCHA_EINVAL,
@@ -984,7 +1328,37 @@ int gemm_grouped(const GemmOperands &op, long long a_rows, long long a_cols, lon
                  TDSCHA_EINVAL, "tc::gemm_grouped: group %d outside its operands", i);
         pb.groups.push_back(g);
     }
-    return dispatch(op, pb, D, ldd, st, err);
+    return 0;
+}
+
+int gemm_grouped(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
+                 const GemmGroup *groups, int n_groups, float *D, long long ldd, cudaStream_t st, unsigned *err) {
+    TD_CHECK(D != nullptr, TDSCHA_EINVAL, "tc::gemm_grouped: NULL output");
+    Problem pb;
+    TD_TRY(check_groups(op, a_rows, a_cols, b_rows, b_cols, groups, n_groups, ldd, &pb));
+    return dispatch(op, nullptr, pb, D, ldd, st, err);
+}
+
+bool weights_fit(Format fmt, int nprod, int K) {
+    return ceil_div(K, (fmt == FMT_TF32 ? 32 : 64) * default_drain(nprod)) <= 2;
+}
+
+int gemm_grouped_weights(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
+                         const GemmGroup *groups, int n_groups, const WeightsOut &wo, cudaStream_t st, unsigned *err) {
+    Problem pb;
+    TD_TRY(check_groups(op, a_rows, a_cols, b_rows, b_cols, groups, n_groups, wo.N2pc, &pb));
+    TD_CHECK(wo.rho && wo.cw_hi && wo.ab_hi && (op.nprod == 1 || (wo.cw_lo && wo.ab_lo)) && (int)wo.K.size() == n_groups &&
+                 (int)wo.col.size() == n_groups && b_rows == 2LL * wo.Nc && wo.N2pc >= 2 * wo.Nc,
+             TDSCHA_EINVAL, "tc::gemm_grouped_weights: bad arguments");
+    const int kblk = op.fmt == FMT_TF32 ? 32 : 64;
+    for (int i = 0; i < n_groups; ++i) {
+        TD_CHECK(groups[i].N == b_rows && groups[i].b_row == 0 && wo.K[i] >= 0 && wo.K[i] % kblk == 0 && wo.col[i] % kblk == 0 &&
+                     wo.col[i] + (long long)wo.K[i] <= wo.ld && weights_fit(op.fmt, op.nprod, wo.K[i]),
+                 TDSCHA_EINVAL, "tc::gemm_grouped_weights: group %d: K=%d at column %d of %lld", i, wo.K[i], wo.col[i], wo.ld);
+        TD_CHECK(wo.K[i] == 0 || (wo.A_hi && wo.B_hi && (op.nprod == 1 || (wo.A_lo && wo.B_lo))), TDSCHA_EINVAL,
+                 "tc::gemm_grouped_weights: NULL [c|d] operand");
+    }
+    return dispatch(op, &wo, pb, nullptr, wo.N2pc, st, err);
 }
 
 }  // namespace tc

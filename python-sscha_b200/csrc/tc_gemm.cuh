@@ -1,6 +1,7 @@
 // tc_gemm.cuh -- interface of the tcgen05 contraction kernel (tc_gemm.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <vector>
 #include "common.cuh"
 
 namespace tdscha {
@@ -36,6 +37,24 @@ struct GemmGroup {
 // groups of a few tiles each leave no SM idle.
 int gemm_grouped(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
                  const GemmGroup *groups, int n_groups, float *D, long long ldd, cudaStream_t st, unsigned *err);
+
+// [a|b] of every group (columns 2Nc) taken straight to the averages' weights: c and d of the same rows and
+// columns are one more short contraction of the tile (operands A_* (a_rows x ld) and B_* (2Nc x ld), columns
+// col[g] .. col[g] + K[g] of group g; K[g] = 0: c = d = 0), and instead of a, b, c, d the weights
+//   Cw = [rho (-d/3 + d4 b/4) / 2 | rho (-c/3 + d4 a/8)],   AB = [-rho a/6 | -rho b/3]
+// are stored, split, in rows of N2pc columns (zero past 2Nc); a group's rows start at row d_off.  fp32
+// arithmetic when Nc is a multiple of 4, FP64 otherwise.
+struct WeightsOut {
+    const void *A_hi, *A_lo, *B_hi, *B_lo;
+    long long ld;
+    std::vector<int> K, col;
+    const double *rho;
+    int Nc, N2pc, d4;
+    void *cw_hi, *cw_lo, *ab_hi, *ab_lo;
+};
+bool weights_fit(Format fmt, int nprod, int K);   // K of [c|d] that the epilogue can take (two chunks)
+int gemm_grouped_weights(const GemmOperands &op, long long a_rows, long long a_cols, long long b_rows, long long b_cols,
+                         const GemmGroup *groups, int n_groups, const WeightsOut &wo, cudaStream_t st, unsigned *err);
 
 // Budget of every bounded wait of later launches (default 4 s), and a one-shot request that the next
 // launch's producers issue no copy (its MMA warps' first wait then runs out): the abort-path test.
