@@ -120,6 +120,12 @@ __global__ void thermal_kernel(const double *w, int n, double T, double *ups, do
     psi[m] = (1.0 + 2.0 * nb) / (2.0 * w[m]);
 }
 
+// factor of every packed pair between Z and W (see SymTables::wfac)
+__global__ void pair_factor_kernel(const double *ups, const int *pmu, const int *pnu, long long P, float *wfac) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p < P) wfac[p] = (float)((pmu[p] == pnu[p] ? 2.0 : 1.0) * ups[pmu[p]] * ups[pnu[p]]);
+}
+
 // (N_sym, d, d) fp64 table -> (N_sym, dp, dp) fp32 zero-padded copies, as given and transposed
 __global__ void pad_sym_kernel(const double *S, int N_sym, int d, int dp, float *P, float *PT) {
     const long long total = (long long)N_sym * dp * dp;
@@ -453,6 +459,7 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
         (rc = dev_alloc((void **)&e->d_bp_c, e->bp_c.size() * sizeof(int), &acc)) ||
         (rc = dev_alloc((void **)&e->d_pair_mu, e->P * sizeof(int), &acc)) ||
         (rc = dev_alloc((void **)&e->d_pair_nu, e->P * sizeof(int), &acc)) ||
+        (rc = dev_alloc((void **)&e->wfac, e->P * sizeof(float), &acc)) ||
         (rc = dev_alloc((void **)&e->d_err, sizeof(unsigned), &acc)))
         return fail(rc);
     e->base_bytes = acc;
@@ -489,6 +496,7 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
         if (crc) return fail(crc);
     }
     thermal_kernel<<<ceil_div(n, 128), 128>>>(e->w, n, T, e->ups, e->psi);
+    pair_factor_kernel<<<ceil_div(e->P, 256), 256>>>(e->ups, e->d_pair_mu, e->d_pair_nu, e->P, e->wfac);
     for (int b = 0; b < n_blocks; ++b) {
         const long long dp = (dim[b] + 3) & ~3;
         pad_sym_kernel<<<grid_for((long long)N_sym * dp * dp), 256>>>(e->sym + e->blk_sym_off[b], N_sym, dim[b], (int)dp,
@@ -528,7 +536,7 @@ int ensemble_destroy(tdscha_ensemble *e) {
     cudaSetDevice(e->device);
     cudaDeviceSynchronize();
     void *ps[] = {e->X, e->Y, e->G, e->Xt, e->rho, e->w, e->ups, e->psi, e->sym, e->symP, e->symPT, e->d_offP, e->d_blk_start, e->d_blk_dim,
-                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->ws.base,
+                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->ws.base,
                   e->vjp_ws.base, e->YX, e->chunk_ops.base, e->XGT, e->d_static_lam, e->Rrow, e->rot_ws.base};
     for (void *p : ps)
         if (p) cudaFree(p);
@@ -865,9 +873,10 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
     const FreqTables &ft = *e->freq;
     const SymCosets *cs = e->cosets;
     const int n_cos = cs->n_cos, sub = cs->sub, nC = ft.n_class;
-    // fold partials: Jf representatives per fold CTA (eight partials of 6 at 48 representatives), so
-    // that each CTA reuses its W block over several representatives
-    const int Jf = std::max(1, ceil_div(n_cos, 8));
+    // fold partials: Jf representatives per fold CTA.  Few partials keep the reduction short, but a CTA walks
+    // its representatives one after the other: with few vectors more and shorter CTAs fill the SMs (2 vectors on
+    // 4x4x4, partials of 6 -> 2 representatives: fold kernels 413 -> 273 us).
+    const int Jf = std::max(1, ceil_div(n_cos, nb >= 8 ? 8 : (nb >= 4 ? 16 : 24)));
     const int nf_total = ceil_div(n_cos, Jf);
     const size_t es = format_bytes(fmt);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -980,7 +989,7 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
         TD_TRY(rotate_mats(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Ys, rtmp, Ysr, true, st));
         TD_TRY(rotate_rows_of(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, R1, R1r, true, st));
     }
-    SymTables tr{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, cs->repP, cs->repPT, cs->d_offRep};
+    SymTables tr{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, cs->repP, cs->repPT, cs->d_offRep, e->wfac};
     SymTables t64{cs->repS, cs->d_offRepS, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, nullptr, nullptr, nullptr};
     int n_classes = 0;
     for (int m = 1; m <= SYM_MT_MAX; ++m) n_classes += e->pairs.count[m] > 0 ? 1 : 0;
@@ -1226,7 +1235,7 @@ int perturb_average_device(tdscha_ensemble *e, int nb, const double *R1, const d
         R1 = R1r;
     }
 
-    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP};
+    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP, e->wfac};
     SymTables tr = t;   // the coset representatives' tables
     if (use_cos) {
         tr.symP = e->cosets->repP;
@@ -1627,7 +1636,7 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
     vjp_cotangent_kernel<<<grid_for((long long)nb * n * n), 256, 0, st>>>(nb, n, fbar, Dbar, e->ups, Rq, Dq);
     TD_CUDA(cudaGetLastError());
 
-    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP};
+    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP, e->wfac};
     bool first = true;
     for (int j0 = 0; j0 < e->N_sym; j0 += Jc) {
         const int nj = std::min(Jc, e->N_sym - j0);
@@ -1762,7 +1771,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     TD_CUDA(cudaMemsetAsync(colsum, 0, 8 * (size_t)N, st));
     vjp_cotangent_kernel<<<grid_for((long long)nb * n * n), 256, 0, st>>>(nb, n, fbar, Dbar, e->ups, Rq, Dq);
     TD_CUDA(cudaGetLastError());
-    SymTables tr{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, cs->repP, cs->repPT, cs->d_offRep};
+    SymTables tr{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, cs->repP, cs->repPT, cs->d_offRep, e->wfac};
     SymTables t64{cs->repS, cs->d_offRepS, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, nullptr, nullptr, nullptr};
     bool first = true;
     for (int p0 = 0; p0 < n_cos; p0 += ncj) {
@@ -1951,7 +1960,7 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
     vjp_cotangent_kernel<<<grid_for((long long)nb * n * n), 256, 0, st>>>(nb, n, fbar, Dbar, e->ups, Rq, Dq);
     TD_CUDA(cudaGetLastError());
 
-    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP};
+    SymTables t{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, e->symP, e->symPT, e->d_offP, e->wfac};
     bool first = true;
     for (int j0 = 0; j0 < e->N_sym; j0 += Jc) {
         const int nj = std::min(Jc, e->N_sym - j0);

@@ -91,6 +91,7 @@ struct tdscha_ensemble {
     double *rho = nullptr, *w = nullptr, *ups = nullptr, *psi = nullptr, *sym = nullptr;
     float *symP = nullptr, *symPT = nullptr;       // padded fp32 symmetry tables (as given, transposed)
     long long *d_offP = nullptr;                   // block offsets into symP / symPT
+    float *wfac = nullptr;                         // per packed pair: ups_mu ups_nu (2 on the diagonal), fp32
     int *d_blk_start = nullptr, *d_blk_dim = nullptr, *d_blocks_ids = nullptr, *d_bp_b = nullptr, *d_bp_c = nullptr;
     long long *d_blk_sym_off = nullptr;
     int *d_pair_mu = nullptr, *d_pair_nu = nullptr;

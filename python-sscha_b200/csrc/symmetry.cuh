@@ -30,6 +30,8 @@ struct SymTables {
     // starting at element offP[b]
     const float *symP, *symPT;
     const long long *offP;
+    // per packed pair: ups_mu ups_nu (2 on the diagonal) in fp32, the factor between Z and W of the mixed-mode fold
+    const float *wfac = nullptr;
     // tensor-core (tcgen05) transform / fold of the bf16 formats (symmetry_umma.cu), when built
     SymUmma *umma = nullptr;
     const int *blocks_ids = nullptr;   // block of each mode (device)
