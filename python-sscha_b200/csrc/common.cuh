@@ -89,6 +89,17 @@ __device__ __forceinline__ float tf32_round(float f) {
     return __uint_as_float(r);
 }
 
+// Correctly rounded x / d from the rounded reciprocal of d: a product, its exact remainder and a
+// correction (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990,
+// theorem on quotients from a correctly rounded reciprocal); three FP64 instructions instead of a division.
+__device__ __forceinline__ double div_by(double x, double d, double r) {   // r = 1 / d, correctly rounded
+    const double q = x * r;
+    const double c = __fma_rn(__fma_rn(-d, q, x), r, q);
+    return isfinite(q) ? c : q;
+}
+template <int D>
+__device__ __forceinline__ double div_const(double x) { return div_by(x, (double)D, 1.0 / D); }
+
 // Store x (FP64) into an operand slot of the given format: hi (and lo when lo != nullptr).
 __device__ __forceinline__ void store_split(Format fmt, void *hi, void *lo, long long idx, double x) {
     if (fmt == FMT_F64) {

@@ -1408,46 +1408,89 @@ __global__ void vjp_coef_kernel(long long M, int N, long long ld, const double *
     }
 }
 
-// colsum[i] += sum_r BR[r][i]
-__global__ void vjp_colsum_kernel(long long M, int N, const double *__restrict__ BR, double *__restrict__ colsum) {
+// part[s][i] = sum of BR[r][i] over the rows r of slice s, then colsum[i] += sum_s part[s][i]: the slices fill the SMs (one
+// thread per configuration over all 2688 rows took 261 us, 107 MB of BR), in a fixed order.
+constexpr int COLSUM_SLICES = 48;
+__global__ void vjp_colsum_kernel(long long M, int N, const double *__restrict__ BR, double *__restrict__ part) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const long long per = (M + COLSUM_SLICES - 1) / COLSUM_SLICES, r0 = blockIdx.y * per, r1 = min(M, r0 + per);
+    double s = 0.0;
+#pragma unroll 8
+    for (long long r = r0; r < r1; ++r) s += BR[r * N + i];
+    part[(long long)blockIdx.y * N + i] = s;
+}
+__global__ void vjp_colsum_add_kernel(int N, const double *__restrict__ part, double *__restrict__ colsum) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     double s = 0.0;
-    for (long long r = 0; r < M; ++r) s += BR[r * N + i];
+#pragma unroll 8
+    for (int k = 0; k < COLSUM_SLICES; ++k) s += part[(long long)k * N + i];
     colsum[i] += s;
+}
+static int vjp_colsum(long long M, int N, const double *BR, double *part, double *colsum, cudaStream_t st) {
+    vjp_colsum_kernel<<<dim3((unsigned)ceil_div(N, 256), COLSUM_SLICES), 256, 0, st>>>(M, N, BR, part);
+    vjp_colsum_add_kernel<<<ceil_div(N, 256), 256, 0, st>>>(N, part, colsum);
+    TD_CUDA(cudaGetLastError());
+    return 0;
 }
 
 // gbar_i += d/dg_i sum_p Vbar[i][p] V[N+i][p] with V[N+i][(mu nu)] = x_mu g_nu + x_nu g_mu off the
-// diagonal and x_mu g_mu on it; one CTA per i, one warp per row mu of the packed triangle
+// diagonal and x_mu g_mu on it; one CTA per i, one warp per row mu of the packed triangle, 192 columns at a time: a
+// lane keeps the sums of its 6 columns in registers over all of the warp's rows (loads of a row are independent),
+// the row's own sum is reduced once.  (One shared-memory FP64 atomic per entry took 270 us for 12720 pairs x 5000
+// configurations, four rows' sums reduced together in a warp per 32 columns 368, this 154 us.)
+constexpr int MV_K = 6, MV_COLS = 32 * MV_K, MV_WARPS = 8;
 template <typename T>
-__global__ void vjp_matvec_kernel(int N, int n, long long Kp, long long np, const T *__restrict__ Vbar,
-                                  const double *__restrict__ X, T *__restrict__ gbar) {
-    extern __shared__ double gs[];
+__global__ void __launch_bounds__(32 * MV_WARPS, 6) vjp_matvec_kernel(int N, int n, long long Kp, long long np, const T *__restrict__ Vbar,
+                                                                   const double *__restrict__ X, T *__restrict__ gbar) {
+    extern __shared__ double gs[];   // n row sums, x (n), column sums of the warps (MV_WARPS x MV_COLS)
+    double *xs = gs + n, *cs = xs + n;
     const int i = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const double *x = X + (long long)i * n;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const T *vb = Vbar + (long long)i * Kp;
-    for (int m = threadIdx.x; m < n; m += blockDim.x) gs[m] = 0.0;
-    __syncthreads();
-    for (int mu = warp; mu < n; mu += nw) {
-        const long long row = (long long)mu * n - ((long long)mu * (mu - 1)) / 2 - mu;   // + nu gives pair(mu, nu)
-        const double xm = x[mu];
-        double own = 0.0;
-        for (int nu = mu + lane; nu < n; nu += 32) {
-            const double v = (double)vb[row + nu];
-            if (nu == mu) {
-                own += v * xm;   // V[N+i, (mu mu)] = x_mu g_mu
-            } else {
-                own += v * x[nu];
-                atomicAdd(&gs[nu], v * xm);
+    for (int m = threadIdx.x; m < n; m += blockDim.x) {
+        gs[m] = 0.0;
+        xs[m] = X[(long long)i * n + m];
+    }
+    for (int c0 = 0; c0 < n; c0 += MV_COLS) {
+        __syncthreads();
+        double col[MV_K];
+#pragma unroll
+        for (int k = 0; k < MV_K; ++k) col[k] = 0.0;
+        for (int mu = warp; mu < min(n, c0 + MV_COLS); mu += MV_WARPS) {
+            const T *row = vb + ((long long)mu * n - ((long long)mu * (mu - 1)) / 2 - mu);   // + nu gives pair(mu, nu)
+            const double xm = xs[mu];
+            double own = 0.0;
+            T v[MV_K];
+#pragma unroll
+            for (int k = 0; k < MV_K; ++k) {
+                const int nu = c0 + 32 * k + lane;
+                v[k] = nu < n && nu >= mu ? row[nu] : T(0);
             }
+#pragma unroll
+            for (int k = 0; k < MV_K; ++k) {
+                const int nu = c0 + 32 * k + lane;
+                own += (double)v[k] * xs[min(nu, n - 1)];     // V[N+i, (mu mu)] = x_mu g_mu: the diagonal once
+                if (nu != mu) col[k] += (double)v[k] * xm;
+            }
+            for (int o = 16; o > 0; o >>= 1) own += __shfl_down_sync(0xffffffffu, own, o);
+            if (lane == 0) gs[mu] += own;                 // this warp's row
         }
-        for (int o = 16; o > 0; o >>= 1) own += __shfl_down_sync(0xffffffffu, own, o);
-        if (lane == 0) atomicAdd(&gs[mu], own);
+#pragma unroll
+        for (int k = 0; k < MV_K; ++k) cs[warp * MV_COLS + 32 * k + lane] = col[k];
+        __syncthreads();
+        for (int c = threadIdx.x; c < MV_COLS && c0 + c < n; c += blockDim.x) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < MV_WARPS; ++w) s += cs[w * MV_COLS + c];
+            gs[c0 + c] += s;
+        }
     }
     __syncthreads();
     for (int m = threadIdx.x; m < n; m += blockDim.x) gbar[(long long)i * np + m] = (T)((double)gbar[(long long)i * np + m] + gs[m]);
 }
+static size_t mv_smem(int n) { return (2 * (size_t)n + MV_WARPS * MV_COLS) * sizeof(double); }
 
 template <typename T>
 __global__ void vjp_final_kernel(int N, int n, long long np, double norm, const double *__restrict__ rho,
@@ -1591,8 +1634,8 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
     const int N = e->N, n = e->n;
     const long long Kp = e->Kp, np = e->np, ld1 = round_up(e->N2, 4);
     // memory plan: fixed buffers, then per symmetry row (M = nb * Jc rows, Mp = M rounded to 64)
-    const size_t fixed = 4 * ((size_t)N * Kp + 2 * (size_t)N * np) + 8 * ((size_t)N + (size_t)nb * n + (size_t)nb * n * n) +
-                         16 * 256;
+    const size_t fixed = 4 * ((size_t)N * Kp + 2 * (size_t)N * np) +
+                         8 * ((size_t)N * (1 + COLSUM_SLICES) + (size_t)nb * n + (size_t)nb * n * n) + 17 * 256;
     const size_t per_row = es * nh * (4 * (size_t)Kp + 4 * (size_t)np + 4 * (size_t)N) + 4 * 4 * (size_t)ld1 + 8 * (size_t)N;
     int Jc = e->N_sym;
     if (e->vjp_ws.bytes < fixed + per_row * (size_t)round_up((long long)nb * Jc, 64) + 64 * 256) {
@@ -1616,6 +1659,7 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
     float *Vbar = static_cast<float *>(take(4 * (size_t)N * Kp));
     float *gbar = static_cast<float *>(take(4 * (size_t)N * np)), *ypart = static_cast<float *>(take(4 * (size_t)N * np));
     double *colsum = static_cast<double *>(take(8 * (size_t)N));
+    double *colpart = static_cast<double *>(take(8 * (size_t)N * COLSUM_SLICES));
     double *Rq = static_cast<double *>(take(8 * (size_t)nb * n)), *Dq = static_cast<double *>(take(8 * (size_t)nb * n * n));
     auto pair_of = [&](size_t count) {
         void *h = take(count * es);
@@ -1672,12 +1716,11 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
         TD_TRY(gemm_abt(e, fmt, nprod, K2.first, K2.second, Mp, N, QT.first, QT.second, Mp, Kp, Mp, Vbar, Kp, st, true));
         TD_TRY(gemm_abt(e, fmt, nprod, K3.first, K3.second, Mp, N, r1T.first, r1T.second, Mp, np, Mp, gbar, np, st, true));
         TD_TRY(gemm_abt(e, fmt, nprod, K4.first, K4.second, Mp, N, phiT.first, phiT.second, Mp, np, Mp, ypart, np, st, true));
-        vjp_colsum_kernel<<<ceil_div(N, 256), 256, 0, st>>>(M, N, BR, colsum);
-        TD_CUDA(cudaGetLastError());
+        TD_TRY(vjp_colsum(M, N, BR, colpart, colsum, st));
         first = false;
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    vjp_matvec_kernel<float><<<N, 256, (size_t)n * sizeof(double), st>>>(N, n, Kp, np, Vbar, e->X, gbar);
+    vjp_matvec_kernel<float><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, Kp, np, Vbar, e->X, gbar);
     vjp_final_kernel<float><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, np, norm, e->rho, e->psi, gbar, ypart, Ybar);
     vjp_rho_kernel<<<1, 256, 0, st>>>(N, norm, e->N_eff, e->rho, colsum, rhobar);
     TD_CUDA(cudaGetLastError());
@@ -1720,7 +1763,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     const FreqOps &co = e->fops[fmt];
     // workspace: fixed part, then per coset (NR = nb * cosets of the chunk, NRp = NR rounded to 64)
     const size_t fixed = as * ((size_t)N * Kq + 2 * (size_t)N * Kmq1 + (size_t)N * e->Kp + 2 * (size_t)N * e->np) +
-                         8 * ((size_t)N + (size_t)nb * n + (size_t)nb * n * n) + 32 * 256;
+                         8 * ((size_t)N * (1 + COLSUM_SLICES) + (size_t)nb * n + (size_t)nb * n * n) + 33 * 256;
     auto per_chunk = [&](int ncj) {
         const size_t NR = (size_t)nb * ncj, NRp = round_up(NR, 64), rows = (size_t)nC * 2 * NR;
         size_t b = 2 * as * (NR * e->Kp + NR * e->np);                      // U, r1, Q, phi
@@ -1752,6 +1795,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     void *VbarQ = take(as * (size_t)N * Kq), *GQ = take(as * (size_t)N * Kmq1), *YQ = take(as * (size_t)N * Kmq1);
     void *Vbar = take(as * (size_t)N * e->Kp), *gbar = take(as * (size_t)N * e->np), *ypart = take(as * (size_t)N * e->np);
     double *colsum = static_cast<double *>(take(8 * (size_t)N));
+    double *colpart = static_cast<double *>(take(8 * (size_t)N * COLSUM_SLICES));
     double *Rq = static_cast<double *>(take(8 * (size_t)nb * n)), *Dq = static_cast<double *>(take(8 * (size_t)nb * n * n));
     void *U = take(as * NRmax * e->Kp), *r1 = take(as * NRmax * e->np), *Q = take(as * NRmax * e->Kp), *phi = take(as * NRmax * e->np);
     auto pair_of = [&](size_t count) { void *h = take(count * es); void *l = lo ? take(count * es) : nullptr; return std::make_pair(h, l); };
@@ -1826,8 +1870,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
             TD_TRY(freq_vjp_coef<float>(ft, sub, (const float *)H, (const float *)Ch, (const float *)HQ, (const float *)Cp, ld1, N,
                                         NR, NRp, apply_d4, true, fmt, Kh, Kl, RT, BR, st));
         }
-        vjp_colsum_kernel<<<ceil_div(N, 256), 256, 0, st>>>(rows, N, BR, colsum);
-        TD_CUDA(cudaGetLastError());
+        TD_TRY(vjp_colsum(rows, N, BR, colpart, colsum, st));
         // transposed contractions over the class rows
         if (f64) {
             std::vector<std::array<long long, 5>> gp, gm;
@@ -1882,13 +1925,13 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     if (f64) {
         TD_TRY(freq_vjp_reconstruct<double>(ft, N, n, e->P, (const double *)VbarQ, (const double *)GQ, (const double *)YQ,
                                             (double *)Vbar, e->Kp, (double *)gbar, (double *)ypart, e->np, st));
-        vjp_matvec_kernel<double><<<N, 256, (size_t)n * sizeof(double), st>>>(N, n, e->Kp, e->np, (const double *)Vbar, e->X, (double *)gbar);
+        vjp_matvec_kernel<double><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, (const double *)Vbar, e->X, (double *)gbar);
         vjp_final_kernel<double><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, (const double *)gbar,
                                                                              (const double *)ypart, Ybar);
     } else {
         TD_TRY(freq_vjp_reconstruct<float>(ft, N, n, e->P, (const float *)VbarQ, (const float *)GQ, (const float *)YQ,
                                            (float *)Vbar, e->Kp, (float *)gbar, (float *)ypart, e->np, st));
-        vjp_matvec_kernel<float><<<N, 256, (size_t)n * sizeof(double), st>>>(N, n, e->Kp, e->np, (const float *)Vbar, e->X, (float *)gbar);
+        vjp_matvec_kernel<float><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, (const float *)Vbar, e->X, (float *)gbar);
         vjp_final_kernel<float><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, (const float *)gbar,
                                                                             (const float *)ypart, Ybar);
     }
@@ -1928,7 +1971,8 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
     }
     const long long ld1 = round_up(e->N2, 4);
     // persistent buffers, then per-chunk rows (M = nb * Jc)
-    const size_t fixed = 8 * ((size_t)N * e->Kp + 2 * (size_t)N * e->np + N + (size_t)nb * n + (size_t)nb * n * n) + 8 * 256;
+    const size_t fixed =
+        8 * ((size_t)N * e->Kp + 2 * (size_t)N * e->np + (size_t)N * (1 + COLSUM_SLICES) + (size_t)nb * n + (size_t)nb * n * n) + 9 * 256;
     const size_t per_row = 8 * (2 * (size_t)e->Kp + 2 * (size_t)e->np + 4 * (size_t)ld1 + 5 * (size_t)N);
     int Jc = e->N_sym;
     if (e->vjp_ws.bytes < fixed + per_row * (size_t)nb * Jc + 16 * 256) {
@@ -1949,7 +1993,7 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
     size_t off = 0;
     auto take = [&](size_t count) { double *p = reinterpret_cast<double *>(W + off); off += (count * 8 + 255) / 256 * 256; return p; };
     double *Vbar = take((size_t)N * e->Kp), *gbar = take((size_t)N * e->np), *ypart = take((size_t)N * e->np);
-    double *colsum = take(N), *Rq = take((size_t)nb * n), *Dq = take((size_t)nb * n * n);
+    double *colsum = take(N), *colpart = take((size_t)N * COLSUM_SLICES), *Rq = take((size_t)nb * n), *Dq = take((size_t)nb * n * n);
     const long long Mmax = (long long)nb * Jc;
     double *B1 = take(Mmax * e->Kp), *Q = take(Mmax * e->Kp), *r1 = take(Mmax * e->np), *phi = take(Mmax * e->np);
     double *D1 = take(Mmax * ld1), *Dcd = take(Mmax * ld1), *DA = take(Mmax * ld1), *DC = take(Mmax * ld1);
@@ -1979,12 +2023,11 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
         TD_TRY(gemm_atb(e, K2, N, Q, e->Kp, M, N, e->Kp, Vbar, e->Kp, true, st));
         TD_TRY(gemm_atb(e, K3, N, r1, e->np, M, N, e->np, gbar, e->np, true, st));
         TD_TRY(gemm_atb(e, K4, N, phi, e->np, M, N, e->np, ypart, e->np, true, st));
-        vjp_colsum_kernel<<<ceil_div(N, 256), 256, 0, st>>>(M, N, BR, colsum);
-        TD_CUDA(cudaGetLastError());
+        TD_TRY(vjp_colsum(M, N, BR, colpart, colsum, st));
         first = false;
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    vjp_matvec_kernel<double><<<N, 256, (size_t)n * sizeof(double), st>>>(N, n, e->Kp, e->np, Vbar, e->X, gbar);
+    vjp_matvec_kernel<double><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, Vbar, e->X, gbar);
     vjp_final_kernel<double><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, gbar, ypart, Ybar);
     vjp_rho_kernel<<<1, 256, 0, st>>>(N, norm, e->N_eff, e->rho, colsum, rhobar);
     TD_CUDA(cudaGetLastError());

@@ -690,51 +690,36 @@ __device__ __forceinline__ void store4_split(Format fmt, void *hi, void *lo, lon
     }
 }
 
-// One CTA row per operand row (grid-stride), threads over quads of configurations.  vec: fp32
-// accumulators, a split format and Nc a multiple of 4 (aligned vector loads and stores).
-template <typename AccT, bool VEC>
-__global__ void __launch_bounds__(256) freq_weights_kernel(const AccT *__restrict__ H, const AccT *__restrict__ Ch, long long ld,
-                                                           const double *__restrict__ rho, long long Nc, int NR, long long rows,
-                                                           const int *__restrict__ cls_real, long long N2pc, int d4, Format fmt,
-                                                           void *Cw_hi, void *Cw_lo, void *AB_hi, void *AB_lo) {
+// One CTA row per operand row (grid-stride), threads over quads of configurations: fp32 accumulators, a split format
+// and Nc a multiple of 4 (aligned vector loads and stores).
+__global__ void __launch_bounds__(256) freq_weights_vec_kernel(const float *__restrict__ H, const float *__restrict__ Ch, long long ld,
+                                                               const double *__restrict__ rho, long long Nc, int NR, long long rows,
+                                                               const int *__restrict__ cls_real, long long N2pc, int d4, Format fmt,
+                                                               void *Cw_hi, void *Cw_lo, void *AB_hi, void *AB_lo) {
     for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
         const long long g = r / (2LL * NR);
         if (r - g * 2LL * NR >= NR && cls_real[g]) continue;   // imaginary row of a real class
-        const AccT *h = H + r * ld, *c = Ch + r * ld;
+        const float *h = H + r * ld, *c = Ch + r * ld;
         const long long o = r * N2pc;
-        if constexpr (VEC) {
-            const float k4 = d4 ? 1.f : 0.f;
-            for (long long i0 = 4LL * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i0 < Nc;
-                 i0 += 4LL * gridDim.x * blockDim.x) {
-                const float4 a = *reinterpret_cast<const float4 *>(h + i0), b = *reinterpret_cast<const float4 *>(h + Nc + i0);
-                const float4 cc = *reinterpret_cast<const float4 *>(c + i0), dd = *reinterpret_cast<const float4 *>(c + Nc + i0);
-                const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-                const float cv[4] = {cc.x, cc.y, cc.z, cc.w}, dv[4] = {dd.x, dd.y, dd.z, dd.w};
-                float half_delta[4], gamma[4], alpha[4], beta[4];
+        const float k4 = d4 ? 1.f : 0.f;
+        for (long long i0 = 4LL * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i0 < Nc; i0 += 4LL * gridDim.x * blockDim.x) {
+            const float4 a = *reinterpret_cast<const float4 *>(h + i0), b = *reinterpret_cast<const float4 *>(h + Nc + i0);
+            const float4 cc = *reinterpret_cast<const float4 *>(c + i0), dd = *reinterpret_cast<const float4 *>(c + Nc + i0);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+            const float cv[4] = {cc.x, cc.y, cc.z, cc.w}, dv[4] = {dd.x, dd.y, dd.z, dd.w};
+            float half_delta[4], gamma[4], alpha[4], beta[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float rh = (float)rho[i0 + e];
-                    gamma[e] = rh * (-cv[e] * (1.f / 3.f) + k4 * av[e] * 0.125f);
-                    half_delta[e] = 0.5f * rh * (-dv[e] * (1.f / 3.f) + k4 * bv[e] * 0.25f);
-                    alpha[e] = -rh * av[e] * (1.f / 6.f);
-                    beta[e] = -rh * bv[e] * (1.f / 3.f);
-                }
-                store4_split(fmt, Cw_hi, Cw_lo, o + i0, half_delta);
-                store4_split(fmt, Cw_hi, Cw_lo, o + Nc + i0, gamma);
-                store4_split(fmt, AB_hi, AB_lo, o + i0, alpha);
-                store4_split(fmt, AB_hi, AB_lo, o + Nc + i0, beta);
+            for (int e = 0; e < 4; ++e) {
+                const float rh = (float)rho[i0 + e];
+                gamma[e] = rh * (-cv[e] * (1.f / 3.f) + k4 * av[e] * 0.125f);
+                half_delta[e] = 0.5f * rh * (-dv[e] * (1.f / 3.f) + k4 * bv[e] * 0.25f);
+                alpha[e] = -rh * av[e] * (1.f / 6.f);
+                beta[e] = -rh * bv[e] * (1.f / 3.f);
             }
-        } else {
-            for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < Nc; i += (long long)gridDim.x * blockDim.x) {
-                const double a = (double)h[i], b = (double)h[Nc + i], cv = (double)c[i], dv = (double)c[Nc + i];
-                const double rh = rho[i];
-                const double gam = rh * (-cv / 3.0 + (d4 ? a / 8.0 : 0.0));
-                const double del = rh * (-dv / 3.0 + (d4 ? b / 4.0 : 0.0));
-                store_split(fmt, Cw_hi, Cw_lo, o + i, 0.5 * del);
-                store_split(fmt, Cw_hi, Cw_lo, o + Nc + i, gam);
-                store_split(fmt, AB_hi, AB_lo, o + i, -rh * a / 6.0);
-                store_split(fmt, AB_hi, AB_lo, o + Nc + i, -rh * b / 3.0);
-            }
+            store4_split(fmt, Cw_hi, Cw_lo, o + i0, half_delta);
+            store4_split(fmt, Cw_hi, Cw_lo, o + Nc + i0, gamma);
+            store4_split(fmt, AB_hi, AB_lo, o + i0, alpha);
+            store4_split(fmt, AB_hi, AB_lo, o + Nc + i0, beta);
         }
         // zero columns past 2Nc (the contractions' K runs to N2pc)
         if (blockIdx.x == 0)
@@ -745,22 +730,71 @@ __global__ void __launch_bounds__(256) freq_weights_kernel(const AccT *__restric
     }
 }
 
+// The same in FP64 arithmetic, any Nc: one thread per configuration and WEIGHT_RB consecutive rows, whose loads overlap.
+// FP64 operands, 31104 rows x 1200 configurations: one row per thread and CTA with FP64 divisions 1015 us, now 353 us (2.4 GB).
+constexpr int WEIGHT_RB = 4;
+template <typename AccT>
+__global__ void __launch_bounds__(256) freq_weights_kernel(const AccT *__restrict__ H, const AccT *__restrict__ Ch, long long ld,
+                                                           const double *__restrict__ rho, int Nc, int NR, int rows,
+                                                           const int *__restrict__ cls_real, int N2pc, int d4, Format fmt,
+                                                           void *Cw_hi, void *Cw_lo, void *AB_hi, void *AB_lo) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double rh = i < Nc ? rho[i] : 0.0;
+    for (int r0 = blockIdx.y * WEIGHT_RB; r0 < rows; r0 += gridDim.y * WEIGHT_RB) {
+        AccT v[WEIGHT_RB][4];
+        bool use[WEIGHT_RB];
+#pragma unroll
+        for (int q = 0; q < WEIGHT_RB; ++q) {
+            const int r = r0 + q, g = r / (2 * NR);
+            use[q] = r < rows && !(r - g * 2 * NR >= NR && cls_real[g]);   // not an imaginary row of a real class
+            if (use[q] && i < Nc) {
+                const AccT *h = H + r * ld + i, *c = Ch + r * ld + i;
+                v[q][0] = h[0]; v[q][1] = h[Nc]; v[q][2] = c[0]; v[q][3] = c[Nc];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < WEIGHT_RB; ++q) {
+            if (!use[q]) continue;
+            const long long o = (long long)(r0 + q) * N2pc;
+            if (i < Nc) {
+                const double a = (double)v[q][0], b = (double)v[q][1], cv = (double)v[q][2], dv = (double)v[q][3];
+                const double gam = rh * (div_const<3>(-cv) + (d4 ? a * 0.125 : 0.0));
+                const double del = rh * (div_const<3>(-dv) + (d4 ? b * 0.25 : 0.0));
+                store_split(fmt, Cw_hi, Cw_lo, o + i, 0.5 * del);
+                store_split(fmt, Cw_hi, Cw_lo, o + Nc + i, gam);
+                store_split(fmt, AB_hi, AB_lo, o + i, div_const<6>(-rh * a));
+                store_split(fmt, AB_hi, AB_lo, o + Nc + i, div_const<3>(-rh * b));
+            }
+            // zero columns past 2Nc (the contractions' K runs to N2pc)
+            if (blockIdx.x == 0)
+                for (int k = 2 * Nc + threadIdx.x; k < N2pc; k += blockDim.x) {
+                    store_split(fmt, Cw_hi, Cw_lo, o + k, 0.0);
+                    store_split(fmt, AB_hi, AB_lo, o + k, 0.0);
+                }
+        }
+    }
+}
+
 }  // namespace
 
 template <typename AccT>
 int freq_weights(const FreqTables &t, const AccT *H, const AccT *Ch, long long ld, const double *rho, long long Nc, int NR,
                  long long N2pc, int d4, Format fmt, void *Cw_hi, void *Cw_lo, void *AB_hi, void *AB_lo, cudaStream_t st) {
     const long long rows = (long long)t.n_class * 2 * NR;
-    const bool vec = sizeof(AccT) == 4 && fmt != FMT_F64 && Nc % 4 == 0 && ld % 4 == 0;
-    const long long per = vec ? ceil_div(Nc, 4) : Nc;
-    const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>(ceil_div(per, 256), 64)),
-                    (unsigned)std::max<long long>(1, std::min<long long>(rows, 65535)));
-    if (vec)
-        freq_weights_kernel<AccT, true><<<grid, 256, 0, st>>>(H, Ch, ld, rho, Nc, NR, rows, t.d_cls_real, N2pc, d4, fmt, Cw_hi,
-                                                              Cw_lo, AB_hi, AB_lo);
-    else
-        freq_weights_kernel<AccT, false><<<grid, 256, 0, st>>>(H, Ch, ld, rho, Nc, NR, rows, t.d_cls_real, N2pc, d4, fmt, Cw_hi,
-                                                               Cw_lo, AB_hi, AB_lo);
+    TD_CHECK(rows < (1LL << 31) && N2pc < (1LL << 30), TDSCHA_EINVAL, "weights of %lld rows x %lld columns", rows, N2pc);
+    if constexpr (sizeof(AccT) == 4) {
+        if (fmt != FMT_F64 && Nc % 4 == 0 && ld % 4 == 0) {
+            const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>(ceil_div(ceil_div(Nc, 4), 256), 64)),
+                            (unsigned)std::max<long long>(1, std::min<long long>(rows, 65535)));
+            freq_weights_vec_kernel<<<grid, 256, 0, st>>>(H, Ch, ld, rho, Nc, NR, rows, t.d_cls_real, N2pc, d4, fmt, Cw_hi, Cw_lo, AB_hi,
+                                                          AB_lo);
+            TD_CUDA(cudaGetLastError());
+            return 0;
+        }
+    }
+    const dim3 grid((unsigned)ceil_div(Nc, 256), (unsigned)std::min<long long>(ceil_div(rows, WEIGHT_RB), 65535));
+    freq_weights_kernel<AccT><<<grid, 256, 0, st>>>(H, Ch, ld, rho, (int)Nc, NR, (int)rows, t.d_cls_real, (int)N2pc, d4, fmt, Cw_hi, Cw_lo,
+                                                    AB_hi, AB_lo);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
@@ -949,12 +983,12 @@ __global__ void __launch_bounds__(256) vjp_coef_class_kernel(const AccT *__restr
                 const long long o = r * ld;
                 const double a = (double)H[o + i], b = (double)H[o + N + i], c = (double)Ch[o + i], d = (double)Ch[o + N + i];
                 const double Ap = (double)HQ[o + i], Bp = (double)HQ[o + N + i], Cq = (double)Cp[o + i], Dq = (double)Cp[o + N + i];
-                const double kk2 = -c / 3.0 + k4 * a / 8.0;
-                v[0] = k4 * Ap / 8.0 - Dq / 3.0;
+                const double kk2 = div_const<3>(-c) + k4 * a * 0.125, a6 = div_const<6>(a);
+                v[0] = k4 * Ap * 0.125 - div_const<3>(Dq);
                 v[1] = kk2;
-                v[2] = -Ap / 6.0;
-                v[3] = -a / 6.0;
-                const double br = 0.5 * (-d / 3.0 + k4 * b / 4.0) * Ap + kk2 * Bp - a / 6.0 * Cq - b / 3.0 * Dq;
+                v[2] = div_const<6>(-Ap);
+                v[3] = -a6;
+                const double br = 0.5 * (div_const<3>(-d) + k4 * b * 0.25) * Ap + kk2 * Bp - a6 * Cq - div_const<3>(b) * Dq;
                 BR[r * N + i] = br * (real_cls ? inv_s_real : inv_s_cplx);
             } else {
                 BR[r * N + i] = 0.0;
@@ -989,22 +1023,34 @@ __global__ void __launch_bounds__(256) vjp_coef_class_kernel(const AccT *__restr
     }
 }
 
+// One thread per pair and LEFT_RB configurations: the pair's columns and factors (24 bytes, more than the 8 bytes of
+// values a configuration reads) are loaded once, and the gathers of the configurations overlap.  12720 pairs x 5000
+// configurations: 1147 us with one configuration at a time and two FP64 divisions an entry, now 199 us.
 template <typename T>
-__global__ void vjp_recon_pairs_kernel(int N, long long P, int Kq, const T *__restrict__ VbarQ, const int *__restrict__ col0,
-                                       const int *__restrict__ col1, const double *__restrict__ pc0, const double *__restrict__ pc1,
-                                       const double *__restrict__ pre, T *__restrict__ Vbar, long long ldv) {
-    for (long long i = blockIdx.y; i < N; i += gridDim.y) {
-        const T *q = VbarQ + i * Kq;
-        for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
-            const int a = col0[p];
-            double v = pc0[p] * (double)q[a] / pre[a];
-            const double k1 = pc1[p];
-            if (k1 != 0.0) {
-                const int b = col1[p];
-                v += k1 * (double)q[b] / pre[b];
-            }
-            Vbar[i * ldv + p] = (T)v;
+__global__ void __launch_bounds__(256) vjp_recon_pairs_kernel(int N, long long P, int Kq, const T *__restrict__ VbarQ,
+                                                              const int *__restrict__ col0, const int *__restrict__ col1,
+                                                              const double *__restrict__ pc0, const double *__restrict__ pc1,
+                                                              const double *__restrict__ pre, T *__restrict__ Vbar, long long ldv) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= P) return;
+    const int a = col0[p], b = col1[p];
+    const double k0 = pc0[p], k1 = pc1[p], da = pre[a], db = k1 != 0.0 ? pre[b] : 1.0, ra = 1.0 / da, rb = 1.0 / db;
+    for (long long i0 = (long long)blockIdx.y * LEFT_RB; i0 < N; i0 += (long long)gridDim.y * LEFT_RB) {
+        const int cnt = (int)min((long long)LEFT_RB, N - i0);
+        T qa[LEFT_RB], qb[LEFT_RB];
+#pragma unroll
+        for (int i = 0; i < LEFT_RB; ++i) {
+            const T *q = VbarQ + (i0 + min(i, cnt - 1)) * Kq;
+            qa[i] = q[a];
+            qb[i] = k1 != 0.0 ? q[b] : T(0);
         }
+#pragma unroll
+        for (int i = 0; i < LEFT_RB; ++i)
+            if (i < cnt) {
+                double v = div_by(k0 * (double)qa[i], da, ra);
+                if (k1 != 0.0) v += div_by(k1 * (double)qb[i], db, rb);
+                Vbar[(i0 + i) * ldv + p] = (T)v;
+            }
     }
 }
 
@@ -1076,7 +1122,8 @@ int freq_vjp_coef(const FreqTables &t, int sub, const AccT *H, const AccT *Ch, c
 template <typename T>
 int freq_vjp_reconstruct(const FreqTables &t, int N, int n, long long P, const T *VbarQ, const T *GQ, const T *YQ, T *Vbar,
                          long long ldv, T *gbar, T *ypart, long long ldg, cudaStream_t st) {
-    vjp_recon_pairs_kernel<T><<<grid_rows(P, N), 256, 0, st>>>(N, P, t.Kq, VbarQ, t.pp_col0, t.pp_col1, t.pp_c0, t.pp_c1, t.pc_re,
+    const dim3 grid((unsigned)ceil_div(P, 256), (unsigned)std::min(ceil_div(N, LEFT_RB), 65535));
+    vjp_recon_pairs_kernel<T><<<grid, 256, 0, st>>>(N, P, t.Kq, VbarQ, t.pp_col0, t.pp_col1, t.pp_c0, t.pp_c1, t.pc_re,
                                                                Vbar, ldv);
     vjp_recon_modes_kernel<T><<<grid1((long long)N * n), 256, 0, st>>>(N, n, t.Kmq, GQ, YQ, t.mode_col, t.mc_sign, t.mc_re, gbar,
                                                                          ypart, ldg);

@@ -272,17 +272,6 @@ struct EpiArgs<true> {
     void *cw_hi, *cw_lo, *ab_hi, *ab_lo;  // rows of N2pc columns; the group's d_off is its first row
 };
 
-// Correctly rounded x / D for D = 3 or 6 with R = 1 / D rounded: a product, its exact remainder and a
-// correction (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990,
-// theorem on quotients from a correctly rounded reciprocal); three FP64 instructions instead of a division.
-template <int D>
-__device__ __forceinline__ double div_const(double x) {
-    constexpr double R = 1.0 / D;
-    const double q = x * R;
-    const double r = __fma_rn(__fma_rn(-(double)D, q, x), R, q);
-    return isfinite(q) ? r : q;
-}
-
 // hi and lo of two weights in the storage format, as bits (bf16: packed into one word each).  Products and
 // differences are rounded one by one.
 template <bool TF32, typename T>
