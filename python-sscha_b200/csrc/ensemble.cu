@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dgemm.cuh"
 #include "ensemble.cuh"
 #include "symmetry.cuh"
 #include "tc_gemm.cuh"
@@ -536,7 +537,7 @@ int ensemble_destroy(tdscha_ensemble *e) {
     cudaSetDevice(e->device);
     cudaDeviceSynchronize();
     void *ps[] = {e->X, e->Y, e->G, e->Xt, e->rho, e->w, e->ups, e->psi, e->sym, e->symP, e->symPT, e->d_offP, e->d_blk_start, e->d_blk_dim,
-                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->ws.base,
+                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->dg_part, e->ws.base,
                   e->vjp_ws.base, e->YX, e->chunk_ops.base, e->XGT, e->d_static_lam, e->Rrow, e->rot_ws.base};
     for (void *p : ps)
         if (p) cudaFree(p);
@@ -841,9 +842,35 @@ static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_t
     return L;
 }
 
-// C (row-major) (+)= A . B^T for every group, FP64 (cuBLAS DGEMM per group)
+// Scratch of the grouped FP64 kernel, once per ensemble and never moved (captured graphs hold its address).  Without
+// it (first call under capture, no memory left) the contractions are not split.
+static int ensure_dg_part(tdscha_ensemble *e, cudaStream_t st) {
+    if (e->dg_part) return 0;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TD_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return 0;
+    void *p = nullptr;
+    if (cudaMalloc(&p, dgemm_part_bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    e->dg_part = p;
+    TD_CUDA(cudaMemsetAsync(p, 0, DGEMM_COUNT_BYTES, st));
+    return 0;
+}
+
+// C (row-major) (+)= A . B^T for every group, FP64.  Groups of up to 2 GF on average go through the grouped kernel of
+// dgemm.cu, larger ones through one cuBLAS DGEMM each, which comes closer to the FP64 peak ([a|b] on 3x3x3, library
+// and grouped kernel, us: 0.66 GF a class 770 and 683, 2.6 GF 2588 and 2489 (Z: 2510 and 2601), 6.6 GF 5736 and 6527).
+constexpr double DG_FLOPS = 2e9;
 static int gemm_groups_f64(tdscha_ensemble *e, const std::vector<tc::GemmGroup> &gs, const double *A, long long lda,
                            const double *B, long long ldb, double *C, long long ldc, bool accumulate, cudaStream_t st) {
+    double flops = 0.0;
+    for (const auto &g : gs) flops += 2.0 * g.M * g.N * g.K;
+    if (flops <= DG_FLOPS * gs.size() && dgemm_fits(A, lda, B, ldb, gs)) {
+        TD_TRY(ensure_dg_part(e, st));
+        return dgemm_grouped(A, lda, B, ldb, gs, C, ldc, accumulate, e->dg_part, st);
+    }
     const double one = 1.0, beta = accumulate ? 1.0 : 0.0;
     cublasSetStream(e->cublas, st);
     for (const auto &g : gs) {

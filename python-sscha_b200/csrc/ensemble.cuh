@@ -100,6 +100,7 @@ struct tdscha_ensemble {
     tdscha::Workspace ws;
     tdscha::Workspace vjp_ws;                      // workspace of the averages' VJP
     tdscha::Workspace chunk_ops;                   // operands of one configuration chunk (large ensembles)
+    void *dg_part = nullptr;                       // scratch of the split FP64 contractions (dgemm.cuh), built by the first
     tdscha::AvgPlan plan;                          // chunking plan of the last averages call
     double *YX = nullptr;                          // [Y; X~] (2N x np), FP64, built by the first VJP
     double *XGT = nullptr;                         // [X^T; G^T] (2n x N), FP64, built by the first operand build
