@@ -9,8 +9,8 @@
 // Systems run on their own streams, forked from and joined back into the caller's stream, so the
 // small systems' kernels fill the SMs the large system's contraction leaves idle.  With use_graph
 // the first two steps run eagerly (they tune the contraction tiles, allocate the workspaces and fix
-// the chunking plans) and all remaining steps of all systems are captured into one CUDA graph that
-// is launched once: the rest of the run is a single launch from the host.
+// the chunking plans) and one step of all systems is captured into a CUDA graph that is launched once
+// for every remaining step (the step counts itself on the device, so all steps are the same graph).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -80,6 +80,7 @@ __global__ void run_rotate_kernel(int nc, long long len, double *__restrict__ qp
 }
 
 struct SysWork {
+    void *base = nullptr;       // one allocation for everything below
     double *out = nullptr;      // (2 nc, len) apply output
     double *next = nullptr;     // (2 nc, len) q', p'
     double *sc_out = nullptr;   // (nc, 4)
@@ -101,13 +102,7 @@ struct RunState {
         for (SysWork &s : w)
             if (s.stream) cudaStreamSynchronize(s.stream);   // nothing in flight uses the buffers below
         for (SysWork &s : w) {
-            cudaFree(s.out);
-            cudaFree(s.next);
-            cudaFree(s.sc_out);
-            cudaFree(s.apply_work);
-            cudaFree(s.lz);
-            cudaFree(s.counter);
-            cudaFree(s.done);
+            cudaFree(s.base);
             if (s.joined) cudaEventDestroy(s.joined);
         }
         if (fork) cudaEventDestroy(fork);
@@ -206,18 +201,24 @@ int lanczos_run_device(int ns, const tdscha_run_system *sys, int n_steps, int us
         const size_t n = s.ens->n;
         TD_TRY(run_stream(s.ens->device, i, &w.stream));
         TD_CUDA(cudaEventCreateWithFlags(&w.joined, cudaEventDisableTiming));
-        TD_CUDA(cudaMalloc(&w.out, (size_t)nb * len * sizeof(double)));
-        TD_CUDA(cudaMalloc(&w.next, (size_t)nb * len * sizeof(double)));
-        TD_CUDA(cudaMalloc(&w.sc_out, (size_t)nc * 4 * sizeof(double)));
         w.apply_bytes = (size_t)nb * (2 * n + 2 * n * n) * sizeof(double);
-        TD_CUDA(cudaMalloc(&w.apply_work, w.apply_bytes));
         w.lz_bytes = lanczos_scratch_bytes(nc);
-        TD_CUDA(cudaMalloc(&w.lz, w.lz_bytes));
-        TD_CUDA(cudaMalloc(&w.counter, sizeof(int)));
-        TD_CUDA(cudaMalloc(&w.done, nc * sizeof(int)));
-        TD_CUDA(cudaMemset(w.done, 0, nc * sizeof(int)));
+        size_t off = 0;
+        auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) / 256 * 256; return o; };
+        const size_t o_out = take((size_t)nb * len * sizeof(double)), o_next = take((size_t)nb * len * sizeof(double)),
+                     o_sc = take((size_t)nc * 4 * sizeof(double)), o_work = take(w.apply_bytes), o_lz = take(w.lz_bytes),
+                     o_done = take((nc + 1) * sizeof(int));
+        TD_CUDA(cudaMalloc(&w.base, off));
+        uint8_t *base = static_cast<uint8_t *>(w.base);
+        w.out = reinterpret_cast<double *>(base + o_out);
+        w.next = reinterpret_cast<double *>(base + o_next);
+        w.sc_out = reinterpret_cast<double *>(base + o_sc);
+        w.apply_work = reinterpret_cast<double *>(base + o_work);
+        w.lz = reinterpret_cast<double *>(base + o_lz);
+        w.done = reinterpret_cast<int *>(base + o_done);
+        w.counter = w.done + nc;
+        TD_CUDA(cudaMemsetAsync(w.done, 0, (nc + 1) * sizeof(int), st));   // before the fork of the first step
         for (int c = nc; c < nb; ++c) w.tr.mask |= 1ull << c;
-        TD_CUDA(cudaMemset(w.counter, 0, sizeof(int)));
     }
     // profiling events cannot be read back from graph replays: off for the run
     std::vector<bool> prof_on(ns);
@@ -233,18 +234,19 @@ int lanczos_run_device(int ns, const tdscha_run_system *sys, int n_steps, int us
         }
     } restore{sys, prof_on};
 
-    const int eager = use_graph ? std::min(n_steps, 2) : n_steps;
+    // The graph pays from three replays on: it is built while the eager steps run, and a step queued call by call takes 45 us
+    // more where the host is the slower side (one chain on 2x2x2, N = 2000, FP64: 5 steps 1.74 ms either way, 12 steps
+    // 4.12 eagerly and 3.81 with the graph, 100 steps 33.8 and 29.1).  All remaining steps in one graph ran no faster
+    // and cost 0.2 ms a step to build (12 steps 5.50 ms, 100 steps 50.6).
+    const char *env = getenv("TDSCHA_RUN_GRAPH_STEPS");   // steps per graph
+    const int env_steps = env ? atoi(env) : 0;
+    const int eager = use_graph && (env_steps > 0 || n_steps >= 2 + 3) ? std::min(n_steps, 2) : n_steps;
     for (int k = 0; k < eager; ++k) TD_TRY(enqueue_step(ns, sys, rs, n_steps, st));
     if (eager < n_steps) {
-        TD_TRY(check_err_words(ns, sys, st));   // also completes the eager steps
-        // the remaining steps go into as few graphs as possible: `per` consecutive steps of all
-        // systems are captured into one graph (TDSCHA_RUN_GRAPH_STEPS caps it; by default all
-        // remaining steps, i.e. a single graph launch for the rest of the run), and a shorter graph
-        // takes the remainder
+        // `per` consecutive steps of all systems per graph, and a shorter graph for the remainder; built while the
+        // eager steps run
         const int rem = n_steps - eager;
-        const char *env = getenv("TDSCHA_RUN_GRAPH_STEPS");
-        const int cap_steps = env && atoi(env) > 0 ? atoi(env) : rem;
-        const int per = std::min(rem, cap_steps);
+        const int per = std::min(rem, env_steps > 0 ? env_steps : 1);
         auto build = [&](int steps, cudaGraphExec_t *exec) -> int {
             cudaGraph_t graph = nullptr;
             TD_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
@@ -269,6 +271,12 @@ int lanczos_run_device(int ns, const tdscha_run_system *sys, int n_steps, int us
                 cudaGraphExecDestroy(full);
                 return rc;
             }
+        }
+        const int rce = check_err_words(ns, sys, st);   // also completes the eager steps
+        if (rce != 0) {
+            cudaGraphExecDestroy(full);
+            if (tail) cudaGraphExecDestroy(tail);
+            return rce;
         }
         cudaError_t el = cudaSuccess;
         for (int k = 0; k + per <= rem && el == cudaSuccess; k += per) el = cudaGraphLaunch(full, st);
