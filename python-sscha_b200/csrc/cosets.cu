@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "cosets.cuh"
+#include "symmetry.cuh"
 
 namespace tdscha {
 
@@ -322,24 +323,167 @@ __global__ void rotate_rows_kernel(long long rows, int n, int dmax, const double
     }
 }
 
-// the row index of each (n x n) matrix: to_rot out[s+q][c] = sum_q' R_b[q'][q] in[s+q'][c], else
-// out[s+q'][c] = sum_q R_b[q'][q] in[s+q][c]
-__global__ void rotate_cols_kernel(int nb, int n, int dmax, const double *__restrict__ Rrow, const int *__restrict__ blocks_ids,
-                                   const int *__restrict__ blk_start, const int *__restrict__ blk_dim,
-                                   const double *__restrict__ in, double *__restrict__ out, bool to_rot) {
-    const long long nn = (long long)n * n, total = (long long)nb * nn;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const long long k = idx / nn;
-        const long long e = idx - k * nn;
-        const int x = (int)(e / n), c = (int)(e - (long long)x * n);
-        const int b = blocks_ids[x], s = blk_start[b], d = blk_dim[b];
-        const double *A = in + k * nn + c;
-        double acc = 0.0;
-        if (to_rot)
-            for (int y = 0; y < d; ++y) acc += Rrow[(long long)(s + y) * dmax + (x - s)] * A[(long long)(s + y) * n];
-        else
-            for (int y = 0; y < d; ++y) acc += Rrow[(long long)x * dmax + y] * A[(long long)(s + y) * n];
-        out[idx] = acc;
+// One tile of one matrix per CTA (blockIdx.y: the vector), rows and columns a group of whole blocks each (RotTiles), and
+// the vectors in the CTAs after the tiles, one group each.  In (OUT = false): out = R^T A R.  Out: out = R A R^T, where A is
+// read as the fold's partial sums: added up over nf, symmetrised from the upper block triangle and scaled.  The tile, both
+// factors and the product in between stay in shared memory, a thread forms Q x Q outputs at a time; every sum runs over the block of its mode in the order of the index.
+// It replaces a launch per index and per vector array (and the reduction) that read columns of blocks through L2:
+// prologue, epilogue, rotations and reduction of a call, us: 2 vectors on 2x2x2 53 -> 32, 5 on 3x3x3 82 -> 38, 2 on 4x4x4
+// 155 -> 105, 16 on 4x4x4 820 -> 340.
+template <bool OUT, int Q>
+__global__ void __launch_bounds__(512) rotate_tiles_kernel(const RotTiles t, const double *__restrict__ mats,
+                                                           const double *__restrict__ vecs, int nf, double norm,
+                                                           double *__restrict__ out, double *__restrict__ vout) {
+    extern __shared__ double sh[];
+    const int n = t.n, dmax = t.dmax, tid = threadIdx.x, nt = blockDim.x, W = t.width, ld = W | 1;
+    const long long k = blockIdx.y, nn = (long long)n * n;
+    const int tiles = t.n_grp * t.n_grp;
+    if ((int)blockIdx.x >= tiles) {
+        const int s0 = t.grp[blockIdx.x - tiles], s1 = t.grp[blockIdx.x - tiles + 1];
+        for (int i = s0 + tid; i < s1; i += nt) {
+            double v = 0.0;
+            if (OUT) {
+#pragma unroll 8
+                for (int f = 0; f < nf; ++f) v += vecs[(k * nf + f) * n + i];
+                v *= norm;
+            } else {
+                v = vecs[k * n + i];
+            }
+            sh[i - s0] = v;
+        }
+        __syncthreads();
+        for (int x = s0 + tid; x < s1; x += nt) {
+            const int b = t.blocks_ids[x], s = t.blk_start[b], d = t.blk_dim[b];
+            double acc = 0.0;
+            for (int y = 0; y < d; ++y) acc += t.Rrow[OUT ? (long long)x * dmax + y : (long long)(s + y) * dmax + x - s] * sh[s - s0 + y];
+            vout[k * n + x] = acc;
+        }
+        return;
+    }
+    const int gi = blockIdx.x / t.n_grp, gj = blockIdx.x - gi * t.n_grp;
+    const int si = t.grp[gi], wi = t.grp[gi + 1] - si, sj = t.grp[gj], wj = t.grp[gj + 1] - sj;
+    // A, T: wi x wj; R?[y][x]: factor of the y-th mode of x's block in output x; o?, d?: first mode and size of x's block
+    double *A = sh, *T = A + W * ld, *Rj = T + W * ld, *Ri = Rj + dmax * ld;
+    int *oj = reinterpret_cast<int *>(Ri + dmax * ld), *dj = oj + W, *oi = dj + W, *di = oi + W;
+    if (OUT) {
+        // the partial sums hold the upper block triangle; E elements of a thread at a time keep the loads in flight
+        constexpr int E = Q == 1 ? 2 : 6;
+        const bool swap = gi > gj;
+        const int cols = swap ? wi : wj;
+        const double *src = mats + k * nf * nn + (long long)(swap ? sj : si) * n + (swap ? si : sj);
+        for (int i0 = tid; i0 < wi * wj; i0 += E * nt) {
+            const double *p[E];
+            double v[E];
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const int i = min(i0 + q * nt, wi * wj - 1), r = i / cols, c = i - r * cols;
+                const bool mirror = gi == gj && t.blocks_ids[si + r] > t.blocks_ids[sj + c];
+                p[q] = src + (long long)(mirror ? c : r) * n + (mirror ? r : c);
+                v[q] = 0.0;
+            }
+#pragma unroll(Q == 1 ? 8 : 4)
+            for (int f = 0; f < nf; ++f)
+#pragma unroll
+                for (int q = 0; q < E; ++q) v[q] += p[q][f * nn];
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const int i = i0 + q * nt, r = i / cols, c = i - r * cols;
+                if (i < wi * wj) A[swap ? c * ld + r : r * ld + c] = v[q] * norm;
+            }
+        }
+    } else {
+        const double *src = mats + k * nn + (long long)si * n + sj;
+        for (int i = tid; i < wi * wj; i += nt) {
+            const int r = i / wj, c = i - r * wj;
+            A[r * ld + c] = src[(long long)r * n + c];
+        }
+    }
+    auto load = [&](int s0, int w, double *R, int *o, int *d) {
+        for (int x = tid; x < w; x += nt) {
+            const int b = t.blocks_ids[s0 + x];
+            o[x] = t.blk_start[b] - s0;
+            d[x] = t.blk_dim[b];
+        }
+        for (int i = tid; i < w * dmax; i += nt) {   // row m of the table: entries of mode m's block
+            const int m = i / dmax, q = i - m * dmax, b = t.blocks_ids[s0 + m], s = t.blk_start[b] - s0;
+            if (q >= t.blk_dim[b]) continue;
+            const double v = t.Rrow[(long long)(s0 + m) * dmax + q];
+            if (OUT) R[q * ld + m] = v;
+            else R[(m - s) * ld + s + q] = v;
+        }
+    };
+    load(sj, wj, Rj, oj, dj);
+    load(si, wi, Ri, oi, di);
+    __syncthreads();
+    // the columns of a thread: an even split of the tile apart, so that a warp's loads fall side by side
+    const int rg = (wi + Q - 1) / Q, cw = (wj + Q - 1) / Q;
+    for (int it = tid; it < rg * cw; it += nt) {   // the column index
+        const int g = it / cw, r0 = Q * g;
+        int x[Q], r[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            x[q] = min(it - g * cw + q * cw, wj - 1);
+            r[q] = min(r0 + q, wi - 1);
+        }
+        double c[Q][Q] = {};
+        if (oj[x[0]] == oj[x[Q - 1]]) {   // one block
+            const double *f = Rj, *a = A + oj[x[0]];
+            const int d = dj[x[0]];
+            for (int y = 0; y < d; ++y, f += ld, ++a) {
+#pragma unroll
+                for (int p = 0; p < Q; ++p)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) c[p][q] += f[x[q]] * a[r[p] * ld];
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const double *f = Rj + x[q], *a = A + oj[x[q]];
+                const int d = dj[x[q]];
+                for (int y = 0; y < d; ++y, f += ld, ++a)
+#pragma unroll
+                    for (int p = 0; p < Q; ++p) c[p][q] += *f * a[r[p] * ld];
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < Q; ++p)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) T[r[p] * ld + x[q]] = c[p][q];   // past the tile's edge: the edge's value again
+    }
+    __syncthreads();
+    double *o = out + k * nn + (long long)si * n + sj;
+    for (int it = tid; it < rg * cw; it += nt) {   // the row index
+        const int g = it / cw, x0 = Q * g;
+        int x[Q], c[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            c[q] = min(it - g * cw + q * cw, wj - 1);
+            x[q] = min(x0 + q, wi - 1);
+        }
+        double v[Q][Q] = {};
+        if (oi[x[0]] == oi[x[Q - 1]]) {
+            const double *f = Ri, *a = T + oi[x[0]] * ld;
+            const int d = di[x[0]];
+            for (int y = 0; y < d; ++y, f += ld, a += ld) {
+#pragma unroll
+                for (int p = 0; p < Q; ++p)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) v[p][q] += f[x[p]] * a[c[q]];
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < Q; ++p) {
+                const double *f = Ri + x[p], *a = T + oi[x[p]] * ld;
+                const int d = di[x[p]];
+                for (int y = 0; y < d; ++y, f += ld, a += ld)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) v[p][q] += *f * a[c[q]];
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < Q; ++p)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) o[(long long)x[p] * n + c[q]] = v[p][q];
     }
 }
 
@@ -539,14 +683,49 @@ int rotate_rows_of(long long rows, int n, int dmax, const double *Rrow, const in
     return 0;
 }
 
-int rotate_mats(int nb, int n, int dmax, const double *Rrow, const int *blocks_ids, const int *blk_start, const int *blk_dim,
-                const double *in, double *tmp, double *out, bool to_rot, cudaStream_t st) {
-    // column index first (every row of every matrix), then the row index
-    TD_TRY(rotate_rows_of((long long)nb * n, n, dmax, Rrow, blocks_ids, blk_start, blk_dim, in, tmp, to_rot, st));
-    rotate_cols_kernel<<<grid_of((long long)nb * n * n), 256, 0, st>>>(nb, n, dmax, Rrow, blocks_ids, blk_start, blk_dim, tmp, out,
-                                                                       to_rot);
+int rotation_tiles(int n_blocks, const int *blk_start, const int *blk_dim, int dmax, std::vector<int> &grp) {
+    // groups of consecutive blocks no wider than the largest block or 24 modes: small blocks share a tile
+    const int width = std::max(dmax, 24);
+    grp.assign(1, 0);
+    for (int b = 0; b < n_blocks; ++b)
+        if (blk_start[b] + blk_dim[b] - grp.back() > width) grp.push_back(blk_start[b]);
+    grp.push_back(blk_start[n_blocks - 1] + blk_dim[n_blocks - 1]);
+    return width;
+}
+
+template <bool OUT, int Q>
+static int rotate_tiles_q(const RotTiles &t, int nb, const double *mats, const double *vecs, int nf, double norm, double *out,
+                        double *vout, cudaStream_t st) {
+    TD_CHECK(t.width <= DMAX_SUPPORTED, TDSCHA_EINVAL, "degenerate block of %d modes exceeds the supported %d", t.dmax, DMAX_SUPPORTED);
+    constexpr int most = 4 * DMAX_SUPPORTED * (DMAX_SUPPORTED | 1) * (int)sizeof(double) + 4 * DMAX_SUPPORTED * (int)sizeof(int);
+    TD_TRY((allow_smem<rotate_tiles_kernel<OUT, Q>>(most)));
+    const size_t smem = (size_t)2 * (t.width + t.dmax) * (t.width | 1) * sizeof(double) + 4 * t.width * sizeof(int);
+    for (int k0 = 0; k0 < nb; k0 += 65535) {
+        const long long o = (long long)k0 * t.n, on = o * t.n;
+        rotate_tiles_kernel<OUT, Q><<<dim3((unsigned)(t.n_grp * t.n_grp + t.n_grp), (unsigned)std::min(nb - k0, 65535)), 512, smem, st>>>(
+            t, mats + (OUT ? nf : 1) * on, vecs + (OUT ? nf : 1) * o, nf, norm, out + on, vout + o);
+    }
     TD_CUDA(cudaGetLastError());
     return 0;
+}
+
+// outputs of a thread: 4 x 4 move a quarter of the operands through shared memory, but leave a small tile's CTA with a
+// warp or two of work (2 vectors on 2x2x2, tiles of 24: the rotation in 14.4 us with 4 x 4, 7.3 with one; 5 vectors on 3x3x3,
+// tiles of 36: 12.7 with 4 x 4, 16.7 with 2 x 2)
+template <bool OUT>
+static int rotate_tiles(const RotTiles &t, int nb, const double *mats, const double *vecs, int nf, double norm, double *out,
+                        double *vout, cudaStream_t st) {
+    const auto run = t.width > 32 ? rotate_tiles_q<OUT, 4> : rotate_tiles_q<OUT, 1>;
+    return run(t, nb, mats, vecs, nf, norm, out, vout, st);
+}
+
+int rotate_in(const RotTiles &t, int nb, const double *A, const double *v, double *out, double *vout, cudaStream_t st) {
+    return rotate_tiles<false>(t, nb, A, v, 1, 1.0, out, vout, st);
+}
+
+int rotate_out(const RotTiles &t, int nb, const double *partD, const double *partF, int nf, double norm, double *out, double *vout,
+               cudaStream_t st) {
+    return rotate_tiles<true>(t, nb, partD, partF, nf, norm, out, vout, st);
 }
 
 int rotate_sym_tables(double *sym_b, int N_sym, int d, const double *Rb, cudaStream_t st) {

@@ -55,9 +55,20 @@ struct SymCosets {
 // to_rot: out = in . R, else out = in . R^T.  Rrow is n x dmax with Rrow[mu][q] = R_b[mu - s_b][q].
 int rotate_rows_of(long long rows, int n, int dmax, const double *Rrow, const int *blocks_ids, const int *blk_start,
                    const int *blk_dim, const double *in, double *out, bool to_rot, cudaStream_t st);
-// (nb x n x n): to_rot: out = R^T A R, else out = R A R^T (tmp: nb x n x n scratch)
-int rotate_mats(int nb, int n, int dmax, const double *Rrow, const int *blocks_ids, const int *blk_start, const int *blk_dim,
-                const double *in, double *tmp, double *out, bool to_rot, cudaStream_t st);
+// Tiles of the rotation of (n x n) matrices: groups of consecutive whole blocks, modes [grp[g], grp[g + 1]).
+struct RotTiles {
+    int n, dmax, n_grp, width;   // width: modes of a group at most
+    const double *Rrow;
+    const int *grp, *blocks_ids, *blk_start, *blk_dim;   // device
+};
+// the groups (n_grp + 1 starts) and their width limit (returned)
+int rotation_tiles(int n_blocks, const int *blk_start, const int *blk_dim, int dmax, std::vector<int> &grp);
+// nb matrices (n x n) and vectors (n) at once: out = R^T A R, vout = v R
+int rotate_in(const RotTiles &t, int nb, const double *A, const double *v, double *out, double *vout, cudaStream_t st);
+// the fold's partial sums (nb x nf x n x n, upper block triangle; nb x nf x n) added up, scaled by norm and
+// rotated back: out = R A R^T, vout = v R^T
+int rotate_out(const RotTiles &t, int nb, const double *partD, const double *partF, int nf, double norm, double *out, double *vout,
+               cudaStream_t st);
 
 // Set-up on the device (ensemble creation): tables (N_sym, d, d) of block b rotated in place,
 // M' = R_b^T M R_b.

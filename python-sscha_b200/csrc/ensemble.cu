@@ -295,6 +295,11 @@ static int setup_cosets(tdscha_ensemble *e, const std::vector<int> &dim, const d
     double *Rblk = nullptr;
     TD_CUDA(cudaMalloc(&e->Rrow, Rrow.size() * sizeof(double)));
     TD_CUDA(cudaMemcpy(e->Rrow, Rrow.data(), Rrow.size() * sizeof(double), cudaMemcpyHostToDevice));
+    std::vector<int> grp;
+    const int width = rotation_tiles(nblk, e->blk_start.data(), dim.data(), dmax, grp);
+    TD_CUDA(cudaMalloc(&e->d_grp, grp.size() * sizeof(int)));
+    TD_CUDA(cudaMemcpy(e->d_grp, grp.data(), grp.size() * sizeof(int), cudaMemcpyHostToDevice));
+    e->rot = RotTiles{n, dmax, (int)grp.size() - 1, width, e->Rrow, e->d_grp, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim};
     TD_CUDA(cudaMalloc(&Rblk, ca.R.size() * sizeof(double)));
     TD_CUDA(cudaMemcpy(Rblk, ca.R.data(), ca.R.size() * sizeof(double), cudaMemcpyHostToDevice));
     // X, Y into the rotated basis (G is free scratch until it is derived from Y)
@@ -538,7 +543,7 @@ int ensemble_destroy(tdscha_ensemble *e) {
     cudaDeviceSynchronize();
     void *ps[] = {e->X, e->Y, e->G, e->Xt, e->rho, e->w, e->ups, e->psi, e->sym, e->symP, e->symPT, e->d_offP, e->d_blk_start, e->d_blk_dim,
                   e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->dg_part, e->ws.base,
-                  e->vjp_ws.base, e->YX, e->chunk_ops.base, e->XGT, e->d_static_lam, e->Rrow, e->rot_ws.base};
+                  e->vjp_ws.base, e->YX, e->chunk_ops.base, e->XGT, e->d_static_lam, e->Rrow, e->d_grp, e->rot_ws.base};
     for (void *p : ps)
         if (p) cudaFree(p);
     for (auto &o : e->ops) free_ops(o);
@@ -610,7 +615,7 @@ static int ensure_operands(tdscha_ensemble *e, Format fmt, bool with_lo, cudaStr
 // Layout of one call's workspace for M = nb * Jc rows.
 struct WsLayout {
     size_t B1_hi, B1_lo, r1_hi, r1_lo, D1, Dcd, Cw_hi, Cw_lo, AB_hi, AB_lo, Z, F, partD, partF;
-    size_t Ucos, r1cos, Ysr, R1r, rtmp;   // coset path and rotated basis (0 when unused)
+    size_t Ucos, r1cos, Ysr, R1r;   // coset path and rotated basis (0 when unused)
     size_t total;
     long long ld1, ldz, ldf;
 };
@@ -649,7 +654,6 @@ static WsLayout layout(const tdscha_ensemble *e, int nb, int Jc, int nf_total, F
     if (e->Rrow) {
         L.Ysr = take((size_t)nb * e->n * e->n * 8);
         L.R1r = take((size_t)nb * e->n * 8);
-        L.rtmp = take((size_t)nb * e->n * e->n * 8);
     }
     L.total = off;
     return L;
@@ -802,7 +806,7 @@ static int ensure_freq_operands(tdscha_ensemble *e, Format fmt, bool lo, cudaStr
 }
 
 struct FreqWs {
-    size_t U, r1, Lab_hi, Lab_lo, Lcd_hi, Lcd_lo, H, Ch, Cw_hi, Cw_lo, AB_hi, AB_lo, O, OF, partD, partF, Ysr, R1r, rtmp;
+    size_t U, r1, Lab_hi, Lab_lo, Lcd_hi, Lcd_lo, H, Ch, Cw_hi, Cw_lo, AB_hi, AB_lo, O, OF, partD, partF, Ysr, R1r;
     size_t total;
     long long ld1, ldz, ldf, N2pc;
 };
@@ -837,7 +841,6 @@ static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_t
     L.partF = take((size_t)nb * nf_total * e->n * 8);
     L.Ysr = take((size_t)nb * e->n * e->n * 8);
     L.R1r = take((size_t)nb * e->n * 8);
-    L.rtmp = take((size_t)nb * e->n * e->n * 8);
     L.total = off;
     return L;
 }
@@ -1008,13 +1011,12 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
     void *Lab_hi = at(L.Lab_hi), *Lab_lo = lo ? at(L.Lab_lo) : nullptr, *Lcd_hi = at(L.Lcd_hi), *Lcd_lo = lo ? at(L.Lcd_lo) : nullptr;
     void *Cw_hi = at(L.Cw_hi), *Cw_lo = lo ? at(L.Cw_lo) : nullptr, *AB_hi = at(L.AB_hi), *AB_lo = lo ? at(L.AB_lo) : nullptr;
     double *partD = static_cast<double *>(at(L.partD)), *partF = static_cast<double *>(at(L.partF));
-    double *Ysr = static_cast<double *>(at(L.Ysr)), *R1r = static_cast<double *>(at(L.R1r)), *rtmp = static_cast<double *>(at(L.rtmp));
+    double *Ysr = static_cast<double *>(at(L.Ysr)), *R1r = static_cast<double *>(at(L.R1r));
     const bool f64 = fmt == FMT_F64;
     const size_t as = f64 ? 8 : 4;
     {
-        StageScope sc(e, ST_OTHER, st, 3);
-        TD_TRY(rotate_mats(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Ys, rtmp, Ysr, true, st));
-        TD_TRY(rotate_rows_of(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, R1, R1r, true, st));
+        StageScope sc(e, ST_OTHER, st, 1);
+        TD_TRY(rotate_in(e->rot, nb, Ys, R1, Ysr, R1r, st));
     }
     SymTables tr{e->sym, e->d_blk_sym_off, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, cs->repP, cs->repPT, cs->d_offRep, e->wfac};
     SymTables t64{cs->repS, cs->d_offRepS, e->d_blk_start, e->d_blk_dim, e->n_blocks, e->n, e->dmax, nullptr, nullptr, nullptr};
@@ -1136,12 +1138,8 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
         }
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    StageScope sc(e, ST_OTHER, st, 4);
-    fold_reduce_kernel<<<grid_for((long long)nb * e->n * e->n), 256, 0, st>>>(partD, partF, nf_total, e->n, nb, e->d_blocks_ids,
-                                                                               norm, Ysr, R1r);
-    TD_CUDA(cudaGetLastError());
-    TD_TRY(rotate_mats(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Ysr, rtmp, d_out, false, st));
-    TD_TRY(rotate_rows_of(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, R1r, f_out, false, st));
+    StageScope sc(e, ST_OTHER, st, 1);
+    TD_TRY(rotate_out(e->rot, nb, partD, partF, nf_total, norm, d_out, f_out, st));
     return 0;
 }
 
@@ -1253,11 +1251,9 @@ int perturb_average_device(tdscha_ensemble *e, int nb, const double *R1, const d
     // inputs into the ensemble's rotated basis
     double *Ysr = e->Rrow ? reinterpret_cast<double *>(W + L.Ysr) : nullptr;
     double *R1r = e->Rrow ? reinterpret_cast<double *>(W + L.R1r) : nullptr;
-    double *rtmp = e->Rrow ? reinterpret_cast<double *>(W + L.rtmp) : nullptr;
     if (e->Rrow) {
-        StageScope sc(e, ST_OTHER, st, 3);
-        TD_TRY(rotate_mats(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Ys, rtmp, Ysr, true, st));
-        TD_TRY(rotate_rows_of(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, R1, R1r, true, st));
+        StageScope sc(e, ST_OTHER, st, 1);
+        TD_TRY(rotate_in(e->rot, nb, Ys, R1, Ysr, R1r, st));
         Ys = Ysr;
         R1 = R1r;
     }
@@ -1367,15 +1363,13 @@ int perturb_average_device(tdscha_ensemble *e, int nb, const double *R1, const d
         }
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    StageScope sc(e, ST_OTHER, st, e->Rrow ? 4 : 1);
-    // in the rotated basis: reduce into the input buffers (free now), then rotate into the outputs
-    double *Dr = e->Rrow ? Ysr : d_out, *fr = e->Rrow ? R1r : f_out;
-    fold_reduce_kernel<<<grid_for((long long)nb * e->n * e->n), 256, 0, st>>>(partD, partF, nf_total, e->n, nb, e->d_blocks_ids,
-                                                                               norm, Dr, fr);
-    TD_CUDA(cudaGetLastError());
+    StageScope sc(e, ST_OTHER, st, 1);
     if (e->Rrow) {
-        TD_TRY(rotate_mats(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Dr, rtmp, d_out, false, st));
-        TD_TRY(rotate_rows_of(nb, e->n, e->dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, fr, f_out, false, st));
+        TD_TRY(rotate_out(e->rot, nb, partD, partF, nf_total, norm, d_out, f_out, st));
+    } else {
+        fold_reduce_kernel<<<grid_for((long long)nb * e->n * e->n), 256, 0, st>>>(partD, partF, nf_total, e->n, nb, e->d_blocks_ids,
+                                                                                   norm, d_out, f_out);
+        TD_CUDA(cudaGetLastError());
     }
     return 0;
 }
@@ -2073,7 +2067,7 @@ int perturb_average_vjp_device(tdscha_ensemble *e, int nb, const double *R1, con
     const int n = e->n;
     const size_t vec = ((size_t)nb * n * 8 + 255) / 256 * 256, mat = ((size_t)nb * n * n * 8 + 255) / 256 * 256;
     const size_t yb = ((size_t)e->N * n * 8 + 255) / 256 * 256;
-    const size_t need = 2 * vec + 3 * mat + yb;
+    const size_t need = 2 * vec + 2 * mat + yb;
     if (e->rot_ws.bytes < need) {
         if (e->rot_ws.base) { TD_CUDA(cudaDeviceSynchronize()); cudaFree(e->rot_ws.base); e->rot_ws = Workspace(); }
         TD_CUDA(cudaMalloc(&e->rot_ws.base, need));
@@ -2082,12 +2076,10 @@ int perturb_average_vjp_device(tdscha_ensemble *e, int nb, const double *R1, con
     uint8_t *W = static_cast<uint8_t *>(e->rot_ws.base);
     double *R1r = reinterpret_cast<double *>(W), *fr = reinterpret_cast<double *>(W + vec);
     double *Ysr = reinterpret_cast<double *>(W + 2 * vec), *Dr = reinterpret_cast<double *>(W + 2 * vec + mat);
-    double *tmp = reinterpret_cast<double *>(W + 2 * vec + 2 * mat), *Yr = reinterpret_cast<double *>(W + 2 * vec + 3 * mat);
+    double *Yr = reinterpret_cast<double *>(W + 2 * vec + 2 * mat);
     const int dmax = e->dmax;
-    TD_TRY(rotate_rows_of(nb, n, dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, R1, R1r, true, st));
-    TD_TRY(rotate_rows_of(nb, n, dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, fbar, fr, true, st));
-    TD_TRY(rotate_mats(nb, n, dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Ys, tmp, Ysr, true, st));
-    TD_TRY(rotate_mats(nb, n, dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Dbar, tmp, Dr, true, st));
+    TD_TRY(rotate_in(e->rot, nb, Ys, R1, Ysr, R1r, st));
+    TD_TRY(rotate_in(e->rot, nb, Dbar, fbar, Dr, fr, st));
     TD_TRY(vjp_in_ensemble_basis(e, nb, R1r, Ysr, apply_d4, fr, Dr, Yr, rhobar, st, precision));
     return rotate_rows_of(e->N, n, dmax, e->Rrow, e->d_blocks_ids, e->d_blk_start, e->d_blk_dim, Yr, Ybar, false, st);
 }

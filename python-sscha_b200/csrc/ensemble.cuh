@@ -116,6 +116,8 @@ struct tdscha_ensemble {
     // sparse: X, Y, G, X~ and the symmetry tables are stored in it, and the averages and their VJP
     // rotate their inputs in and their outputs back.  nullptr: the basis as given.
     double *Rrow = nullptr;                        // n x dmax, Rrow[mu][q] = R_b[mu - s_b][q]
+    int *d_grp = nullptr;                          // mode groups of the rotations' tiles
+    tdscha::RotTiles rot{};
     tdscha::SymCosets *cosets = nullptr;           // factorised symmetry transform / fold (mixed formats)
     tdscha::FreqTables *freq = nullptr;            // character classes of the subgroup (freq.cuh)
     tdscha::FreqOps fops[3];                       // character-basis operands per storage format (resident)
