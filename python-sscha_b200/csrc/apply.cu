@@ -437,10 +437,20 @@ struct CFParams {
     double sign, shift, smearing, modulus;
 };
 
-__global__ void cf_kernel(CFParams prm, const double *a, const double *b, const double *c, int n_w, const double *omega, double *gf) {
-    const int iw = blockIdx.x * blockDim.x + threadIdx.x;
-    if (iw >= n_w) return;
-    const double w = omega[iw];
+// One frequency per thread, 32 threads per block (a grid of a few hundred frequencies then spreads over the SMs).  The chain
+// of coefficients is serial, and a complex division per step made it 300 cycles a step.  With g = P / Q the
+// step g <- 1 / (d - bc g) is (P, Q) <- (Q, d Q - bc P), two dependent FMAs, and one division at the end; both are
+// scaled by a power of two every CF_GROUP steps.  A denominator of zero, or a value that leaves the range of a
+// double within a group, goes through the division per step as written (same infinities and NaN).
+// 100 steps, 500 frequencies: 18.3 -> 8 us (with a group of 4 steps 9).
+constexpr int CF_THREADS = 32, CF_CHUNK = 256, CF_GROUP = 8;
+
+__global__ void __launch_bounds__(CF_THREADS) cf_kernel(CFParams prm, const double *__restrict__ a, const double *__restrict__ b,
+                                                        const double *__restrict__ c, int n_w, const double *__restrict__ omega,
+                                                        double *__restrict__ gf) {
+    __shared__ double2 co[CF_CHUNK];   // (A_i, B_i C_i)
+    const int iw = blockIdx.x * CF_THREADS + threadIdx.x;
+    const double w = omega[min(iw, n_w - 1)];
     const double wsgn = prm.use_wigner ? 1.0 : -1.0;     // a -/+ w^2
     const bool nonsym = (c != nullptr) && (prm.n_c == prm.n_b);
     cuDoubleComplex g;
@@ -468,13 +478,55 @@ __global__ void cf_kernel(CFParams prm, const double *a, const double *b, const 
         const double A = a[prm.n_iter - 1] * prm.sign - prm.sign * prm.shift;
         g = cuCdiv(make_cuDoubleComplex(1.0, 0.0), make_cuDoubleComplex(A + wsgn * w * w, 2 * w * prm.smearing));
     }
-    for (int i = prm.n_iter - 2; i >= 0; --i) {
-        const double A = a[i] * prm.sign - prm.sign * prm.shift;
-        const double B = b[i] * prm.sign;
-        const double C = nonsym ? c[i] * prm.sign : B;
-        cuDoubleComplex den = make_cuDoubleComplex(A + wsgn * w * w, 2 * w * prm.smearing);
-        den = cuCsub(den, cuCmul(make_cuDoubleComplex(B * C, 0.0), g));
-        g = cuCdiv(make_cuDoubleComplex(1.0, 0.0), den);
+    const double ww = wsgn * w * w, di = 2 * w * prm.smearing;
+    double Pr = cuCreal(g), Pi = cuCimag(g), Qr = 1.0, Qi = 0.0;
+    bool plain = prm.n_iter < 2;   // nothing to advance: g stands
+    for (int top = prm.n_iter - 2; top >= 0; top -= CF_CHUNK) {   // steps top, top - 1, ...
+        const int m = min(top + 1, CF_CHUNK);
+        __syncthreads();
+        for (int j = threadIdx.x; j < m; j += CF_THREADS) {
+            const int i = top - j;
+            const double B = b[i] * prm.sign, C = nonsym ? c[i] * prm.sign : B;
+            co[j] = make_double2(a[i] * prm.sign - prm.sign * prm.shift, B * C);
+        }
+        __syncthreads();
+        for (int j0 = 0; j0 < m; j0 += CF_GROUP) {
+#pragma unroll
+            for (int j = 0; j < CF_GROUP; ++j) {
+                if (j0 + j < m) {
+                    const double2 k = co[j0 + j];
+                    const double dr = k.x + ww;
+                    const double nr = fma(dr, Qr, fma(-di, Qi, -(k.y * Pr))), ni = fma(dr, Qi, fma(di, Qr, -(k.y * Pi)));
+                    Pr = Qr;
+                    Pi = Qi;
+                    Qr = nr;
+                    Qi = ni;
+                    plain |= fmax(fabs(nr), fabs(ni)) < 1e-270;
+                }
+            }
+            // the largest part to [1, 2)
+            const double big = fmax(fmax(fabs(Pr), fabs(Pi)), fmax(fabs(Qr), fabs(Qi)));
+            const int e = __double2hiint(big) >> 20;   // biased exponent
+            plain |= !(e > 64 && e < 1984) || isnan(Pr) || isnan(Pi) || isnan(Qr) || isnan(Qi);
+            const double sc = __hiloint2double((2046 - min(max(e, 64), 1984)) << 20, 0);
+            Pr *= sc;
+            Pi *= sc;
+            Qr *= sc;
+            Qi *= sc;
+        }
+    }
+    if (iw >= n_w) return;
+    if (plain) {
+        for (int i = prm.n_iter - 2; i >= 0; --i) {
+            const double A = a[i] * prm.sign - prm.sign * prm.shift;
+            const double B = b[i] * prm.sign;
+            const double C = nonsym ? c[i] * prm.sign : B;
+            cuDoubleComplex den = make_cuDoubleComplex(A + wsgn * w * w, 2 * w * prm.smearing);
+            den = cuCsub(den, cuCmul(make_cuDoubleComplex(B * C, 0.0), g));
+            g = cuCdiv(make_cuDoubleComplex(1.0, 0.0), den);
+        }
+    } else {
+        g = cuCdiv(make_cuDoubleComplex(Pr, Pi), make_cuDoubleComplex(Qr, Qi));
     }
     double re = cuCreal(g), im = cuCimag(g);
     if (prm.use_wigner) re = -re;
@@ -489,7 +541,7 @@ int continued_fraction_device(int n_iter, const double *a, const double *b, cons
     TD_CHECK(n_iter == 1 || (b && n_b >= n_iter - 1), TDSCHA_EINVAL, "need at least n_iter - 1 b coefficients");
     TD_CHECK(!use_terminator || (b && n_b >= 1 && last_average >= 1), TDSCHA_EINVAL, "terminator needs b coefficients");
     CFParams prm{n_iter, n_b, c ? n_c : 0, use_terminator, last_average, use_wigner, reverse_L ? -1.0 : 1.0, shift_value, smearing, modulus};
-    cf_kernel<<<ceil_div(n_w, 128), 128, 0, st>>>(prm, a, b, c, n_w, omega, gf_out);
+    cf_kernel<<<ceil_div(n_w, CF_THREADS), CF_THREADS, 0, st>>>(prm, a, b, c, n_w, omega, gf_out);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
