@@ -101,6 +101,9 @@ struct tdscha_ensemble {
     tdscha::Workspace vjp_ws;                      // workspace of the averages' VJP
     tdscha::Workspace chunk_ops;                   // operands of one configuration chunk (large ensembles)
     void *dg_part = nullptr;                       // scratch of the split FP64 contractions (dgemm.cuh), built by the first
+    cudaStream_t side = nullptr;                   // F's contraction beside Z's
+    cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    int sms = 0;
     tdscha::AvgPlan plan;                          // chunking plan of the last averages call
     double *YX = nullptr;                          // [Y; X~] (2N x np), FP64, built by the first VJP
     double *XGT = nullptr;                         // [X^T; G^T] (2n x N), FP64, built by the first operand build

@@ -1075,7 +1075,7 @@ static int prepare_cfg(const GemmOperands &op, const WeightsOut *wo, const Probl
     // rows x 20000, K <= 2432: 1623 us aligned, 1564 us not; Z (K = 20032) the same either way.
     int k_max = 0;
     for (size_t i = g0; i < g1; ++i) k_max = std::max(k_max, pb.groups[i].K);
-    unsigned *cnt = (sync_ns > 0 && tiles > grid.x && k_max >= 32768) ? counter : nullptr;
+    unsigned *cnt = (sync_ns > 0 && counter && tiles > grid.x && k_max >= 32768) ? counter : nullptr;
     EpiArgs<WEIGHTS> ea{};
     if constexpr (WEIGHTS) {
         CUtensorMap *wa[2] = {SWAP ? &ea.q_hi : &ea.p_hi, SWAP ? &ea.q_lo : &ea.p_lo}, *wb[2] = {SWAP ? &ea.p_hi : &ea.q_hi, SWAP ? &ea.p_lo : &ea.q_lo};
@@ -1234,7 +1234,7 @@ static int launch_tuned(const GemmOperands &op, const WeightsOut *wo, const Prob
     TD_CUDA(cudaStreamIsCapturing(st, &cap));
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     unsigned *counter = nullptr;
-    if (tile_sync_budget_ns() > 0) TD_TRY(tile_sync_counter(dev, st, capturing, &counter));
+    if (op.tile_sync && tile_sync_budget_ns() > 0) TD_TRY(tile_sync_counter(dev, st, capturing, &counter));
     const int stall = g_stall_next.exchange(0);
     const int drain = op.drain_kb > 0 ? op.drain_kb : default_drain(NPROD);
     for (size_t g0 = 0; g0 < pb.groups.size(); g0 += MAX_GROUPS) {
@@ -1261,6 +1261,7 @@ static int launch_tuned(const GemmOperands &op, const WeightsOut *wo, const Prob
         if (!stall) TD_TRY(choose_order(key, cfg, sms, st, !op.accumulate && !capturing, &gp));
         cfg.launch(gp);
         TD_CUDA(cudaGetLastError());
+        if (op.ctas) *op.ctas = std::max(*op.ctas, (int)std::min<long long>(pl.tiles, sms));
     }
     return 0;
 }

@@ -19,6 +19,8 @@ struct GemmOperands {
     long long ldb;
     int drain_kb = 0;   // k-blocks per TMEM chunk drained to fp32 registers (0 = library default)
     bool accumulate = false;   // D += A . B^T instead of D = A . B^T
+    bool tile_sync = true;     // co-resident tiles may wait for one another (bounded) to share operand slices
+    int *ctas = nullptr;       // out: most CTAs of one of the launches
 };
 
 // K must be a multiple of 64 (bf16) or 32 (tf32); operands must be readable up to K columns.
