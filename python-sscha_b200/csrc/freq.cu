@@ -302,12 +302,6 @@ dim3 grid_cols_rows(long long cols, long long rows, int rb) {
     return dim3((unsigned)gx, (unsigned)gy);
 }
 
-dim3 grid_rows(long long cols, long long rows) {
-    const long long gx = std::max<long long>(1, std::min<long long>(ceil_div(cols, 256), 64));
-    const long long gy = std::max<long long>(1, std::min<long long>(rows, 65535));
-    return dim3((unsigned)gx, (unsigned)gy);
-}
-
 // Vq (2Nc x Kq) and VqT (Kq x N2pc) together: one CTA per 64 x 64 tile of (configuration rows,
 // component columns) computes the tile once into shared memory (hi, lo) and writes it row-major and
 // transposed, 128 bytes or more per warp on both sides.  Rows k >= 2Nc (up to N2pc) are zero in VqT.
