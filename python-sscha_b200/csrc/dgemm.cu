@@ -2,12 +2,12 @@
 //
 // The class contractions of a small system are eight or fourteen products of a few 0.1 GF each; one library call per
 // class is bound by its launches (48 kernels per apply on 2x2x2, 8 to 14 us each, twice that where the library splits K).
-// Here a CTA takes one 32- or 64-row x 64-column tile of any class, and a contraction over the configurations (few tiles,
+// Here a CTA takes one 32- or 64-row x 16- or 64-column tile of any class, and a contraction over the configurations (few tiles,
 // long K) is cut into slices of K whose partial tiles the last CTA to finish adds up in slice order (the result does not
 // depend on which one that is).  Four warps, m8n8k4 FP64 tensor instructions, three stages of 16 k in shared memory with
 // 20-double rows: the 8 x 4 fragment reads of a half warp fall on all banks.
-// Measured, us, one library call per class -> this: 2 vectors on 2x2x2, N = 2000: [a|b] 86 -> 42, [c|d] 61 -> 25, Z 121 -> 46,
-// F 101 -> 27; F of 2 vectors on 4x4x4, N = 10000: 912 -> 570.  Large classes come out at 30 TFLOP/s: the FP64 unit, with
+// Measured, us, one library call per class -> this: 2 vectors on 2x2x2, N = 2000: [a|b] 86 -> 42, [c|d] 61 -> 17, Z 121 -> 46,
+// F 101 -> 21; F of 2 vectors on 4x4x4, N = 10000: 912 -> 280.  Large classes come out at 30 TFLOP/s: the FP64 unit, with
 // 10 % lost to what its warps wait for; 16x8x8 instructions and 96-row tiles of 8 warps were no faster.
 #include <algorithm>
 #include <cstdint>
@@ -17,7 +17,7 @@
 namespace tdscha {
 namespace {
 
-constexpr int MAX_G = 64, BN = 64, BK = 16, LDS = BK + 4, STAGES = 3, THREADS = 128;
+constexpr int MAX_G = 64, BK = 16, LDS = BK + 4, STAGES = 3, THREADS = 128;
 constexpr int MAX_CTAS = DGEMM_MAX_CTAS;
 
 struct DGroup {
@@ -36,13 +36,13 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
 
-// BM = 32 or 64 rows; the warps form a 2 x 2 grid, each with BM / 2 x 32 outputs
-template <int BM>
+// BM = 32 or 64 rows; the warps form a 2 x 2 grid (4 x 1 for 16 columns)
+template <int BM, int BN>
 __global__ void __launch_bounds__(THREADS) dgemm_grouped_kernel(const double *__restrict__ A, long long lda, const double *__restrict__ B,
                                                                 long long ldb, double *__restrict__ C, long long ldc,
                                                                 const __grid_constant__ DTable t, double *__restrict__ part,
                                                                 unsigned *__restrict__ count, int accumulate) {
-    constexpr int MI = BM / 16, NI = 4;   // 8 x 8 tiles of a warp
+    constexpr int WN = BN == 16 ? 1 : 2, WR = BM * WN / 4, WC = BN / WN, MI = WR / 8, NI = WC / 8;   // 8 x 8 tiles of a warp
     extern __shared__ __align__(16) double sm[];
     double *As = sm, *Bs = sm + STAGES * BM * LDS;
     int gi = 0;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(THREADS) dgemm_grouped_kernel(const double *__
         if (s < nk) issue(kb0 + s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * 32;
+    const int wm = warp / WN * WR, wn = warp % WN * WC;
     const int fr = lane >> 2, fk = lane & 3;
     for (int k = 0; k < nk; ++k) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(THREADS) dgemm_grouped_kernel(const double *__
     }
 }
 
-template <int BM>
+template <int BM, int BN>
 int launch(const double *A, long long lda, const double *B, long long ldb, const tc::GemmGroup *gs, int n, double *C, long long ldc,
            bool accumulate, void *part, cudaStream_t st) {
     DTable t{};
@@ -178,8 +178,8 @@ int launch(const double *A, long long lda, const double *B, long long ldb, const
     }
     unsigned *count = static_cast<unsigned *>(part);
     constexpr int smem = STAGES * (BM + BN) * LDS * (int)sizeof(double);
-    TD_TRY(allow_smem<dgemm_grouped_kernel<BM>>(smem));
-    dgemm_grouped_kernel<BM><<<dim3((unsigned)tiles, (unsigned)t.slices), THREADS, smem, st>>>(A, lda, B, ldb, C, ldc, t,
+    TD_TRY((allow_smem<dgemm_grouped_kernel<BM, BN>>(smem)));
+    dgemm_grouped_kernel<BM, BN><<<dim3((unsigned)tiles, (unsigned)t.slices), THREADS, smem, st>>>(A, lda, B, ldb, C, ldc, t,
                                                                                             reinterpret_cast<double *>(count + MAX_CTAS), count,
                                                                                             accumulate ? 1 : 0);
     TD_CUDA(cudaGetLastError());
@@ -188,7 +188,7 @@ int launch(const double *A, long long lda, const double *B, long long ldb, const
 
 }  // namespace
 
-size_t dgemm_part_bytes() { return DGEMM_COUNT_BYTES + (size_t)MAX_CTAS * 64 * BN * sizeof(double); }
+size_t dgemm_part_bytes() { return DGEMM_COUNT_BYTES + (size_t)MAX_CTAS * 64 * 64 * sizeof(double); }
 
 bool dgemm_fits(const double *A, long long lda, const double *B, long long ldb, const std::vector<tc::GemmGroup> &gs) {
     bool ok = lda % 2 == 0 && ldb % 2 == 0 && (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) % 16 == 0;
@@ -206,7 +206,13 @@ int dgemm_grouped(const double *A, long long lda, const double *B, long long ldb
         w32 += round_up(g.M, 32) * g.N * g.K;
         w64 += round_up(g.M, 64) * g.N * g.K;
     }
-    const auto run = w64 <= 1.1 * w32 ? launch<64> : launch<32>;
+    // columns per tile: the products over a class's modes (5 to 16 columns) are bound by the rows' stream, and with 64
+    // columns by products that are thrown away (F of 24 vectors on 3x3x3, N = 1200: 350 -> 160 us; 2 vectors on 4x4x4,
+    // N = 10000: 570 -> 280)
+    int nmax = 0;
+    for (const auto &g : gs) nmax = std::max(nmax, g.N);
+    const bool m64 = w64 <= 1.1 * w32;
+    const auto run = nmax <= 16 ? (m64 ? launch<64, 16> : launch<32, 16>) : (m64 ? launch<64, 64> : launch<32, 64>);
     for (size_t i = 0; i < gs.size(); i += MAX_G) {
         const int n = (int)std::min<size_t>(MAX_G, gs.size() - i);
         TD_TRY(run(A, lda, B, ldb, gs.data() + i, n, C, ldc, accumulate, part, st));

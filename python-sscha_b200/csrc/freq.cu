@@ -186,6 +186,7 @@ int build_freq_layout(int n, const std::vector<int> &dim, const std::vector<int>
         int mcnt = 0;
         for (int k : mby_cls[g]) { mcomps[k].col = kmq + mcnt; mcnt += mcomps[k].qb >= 0 ? 2 : 1; }
         out.mcol_cnt.push_back(mcnt ? (int)round_up(mcnt, 64) : 0);
+        out.mcol_use.push_back((int)round_up(mcnt, 16));
         kmq += out.mcol_cnt.back();
         (void)id;
     }
@@ -809,6 +810,7 @@ int freq_tables_create(const FreqLayout &L, FreqTables **out) {
     t->pcol_cnt = L.pcol_cnt;
     t->mcol_off = L.mcol_off;
     t->mcol_cnt = L.mcol_cnt;
+    t->mcol_use = L.mcol_use;
     t->flops_ratio = L.flops_ratio;
     size_t acc = 0;
     int rc = 0;

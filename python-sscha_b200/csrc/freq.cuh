@@ -37,6 +37,7 @@ struct FreqLayout {
     std::vector<int> cls_real;                        // class is a real character
     std::vector<int> pcol_off, pcol_cnt;              // pair columns of each class (padded)
     std::vector<int> mcol_off, mcol_cnt;              // mode columns of each class (padded; 0 when none)
+    std::vector<int> mcol_use;                        // of these, up to the first 16 that hold padding only
     // per pair column: own value = c0 M[mu0, nu0] + c1 M[mu1, nu1] of a symmetric matrix M
     std::vector<int> pc_mu0, pc_nu0, pc_mu1, pc_nu1;
     std::vector<double> pc_c0, pc_c1;
@@ -60,7 +61,7 @@ int build_freq_layout(int n, const std::vector<int> &dim, const std::vector<int>
 // Device copy of the layout tables.
 struct FreqTables {
     int n_class = 0, Kq = 0, Kmq = 0;
-    std::vector<int> cls_real, pcol_off, pcol_cnt, mcol_off, mcol_cnt;
+    std::vector<int> cls_real, pcol_off, pcol_cnt, mcol_off, mcol_cnt, mcol_use;
     int *pc_mu0 = nullptr, *pc_nu0 = nullptr, *pc_mu1 = nullptr, *pc_nu1 = nullptr, *pc_partner = nullptr;
     double *pc_c0 = nullptr, *pc_c1 = nullptr, *pc_re = nullptr, *pc_im = nullptr, *pc_zc = nullptr;
     int *pp_col0 = nullptr, *pp_col1 = nullptr;
