@@ -1571,7 +1571,17 @@ __global__ void __launch_bounds__(32 * MV_WARPS, 6) vjp_matvec_kernel(int N, int
     __syncthreads();
     for (int m = threadIdx.x; m < n; m += blockDim.x) gbar[(long long)i * np + m] = (T)((double)gbar[(long long)i * np + m] + gs[m]);
 }
+// x and the row sums of every mode stay in shared memory, which bounds the modes (13760)
 static size_t mv_smem(int n) { return (2 * (size_t)n + MV_WARPS * MV_COLS) * sizeof(double); }
+constexpr int MV_SMEM_MAX = 227 * 1024;
+
+template <typename T>
+static int vjp_matvec(int N, int n, long long Kp, long long np, const T *Vbar, const double *X, T *gbar, cudaStream_t st) {
+    TD_TRY((allow_smem<vjp_matvec_kernel<T>>(MV_SMEM_MAX)));
+    vjp_matvec_kernel<T><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, Kp, np, Vbar, X, gbar);
+    TD_CUDA(cudaGetLastError());
+    return 0;
+}
 
 template <typename T>
 __global__ void vjp_final_kernel(int N, int n, long long np, double norm, const double *__restrict__ rho,
@@ -1801,7 +1811,7 @@ static int perturb_average_vjp_mixed(tdscha_ensemble *e, int nb, const double *R
         first = false;
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    vjp_matvec_kernel<float><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, Kp, np, Vbar, e->X, gbar);
+    TD_TRY(vjp_matvec<float>(N, n, Kp, np, Vbar, e->X, gbar, st));
     vjp_final_kernel<float><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, np, norm, e->rho, e->psi, gbar, ypart, Ybar);
     vjp_rho_kernel<<<1, 256, 0, st>>>(N, norm, e->N_eff, e->rho, colsum, rhobar);
     TD_CUDA(cudaGetLastError());
@@ -2006,13 +2016,13 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     if (f64) {
         TD_TRY(freq_vjp_reconstruct<double>(ft, N, n, e->P, (const double *)VbarQ, (const double *)GQ, (const double *)YQ,
                                             (double *)Vbar, e->Kp, (double *)gbar, (double *)ypart, e->np, st));
-        vjp_matvec_kernel<double><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, (const double *)Vbar, e->X, (double *)gbar);
+        TD_TRY(vjp_matvec<double>(N, n, e->Kp, e->np, (const double *)Vbar, e->X, (double *)gbar, st));
         vjp_final_kernel<double><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, (const double *)gbar,
                                                                              (const double *)ypart, Ybar);
     } else {
         TD_TRY(freq_vjp_reconstruct<float>(ft, N, n, e->P, (const float *)VbarQ, (const float *)GQ, (const float *)YQ,
                                            (float *)Vbar, e->Kp, (float *)gbar, (float *)ypart, e->np, st));
-        vjp_matvec_kernel<float><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, (const float *)Vbar, e->X, (float *)gbar);
+        TD_TRY(vjp_matvec<float>(N, n, e->Kp, e->np, (const float *)Vbar, e->X, (float *)gbar, st));
         vjp_final_kernel<float><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, (const float *)gbar,
                                                                             (const float *)ypart, Ybar);
     }
@@ -2024,6 +2034,8 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
 static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, const double *Ys, int apply_d4,
                                  const double *fbar, const double *Dbar, double *Ybar, double *rhobar, cudaStream_t st,
                                  int precision) {
+    TD_CHECK(mv_smem(e->n) <= MV_SMEM_MAX, TDSCHA_EINVAL, "the averages' VJP takes at most %d modes (got %d)",
+             (int)(MV_SMEM_MAX / sizeof(double) - MV_WARPS * MV_COLS) / 2, e->n);
     if (e->freq && use_freq_path(e, format_of(precision)) && vjp_freq_enabled()) {
         TD_CHECK(nb > 0, TDSCHA_EINVAL, "nb must be positive");
         TD_CHECK(apply_d4 == 0 || apply_d4 == 1, TDSCHA_EINVAL, "apply_D4 must be 0 or 1 (got %d)", apply_d4);
@@ -2108,7 +2120,7 @@ static int vjp_in_ensemble_basis(tdscha_ensemble *e, int nb, const double *R1, c
         first = false;
     }
     const double norm = 1.0 / (e->N_eff * (double)e->N_sym);
-    vjp_matvec_kernel<double><<<N, 32 * MV_WARPS, mv_smem(n), st>>>(N, n, e->Kp, e->np, Vbar, e->X, gbar);
+    TD_TRY(vjp_matvec<double>(N, n, e->Kp, e->np, Vbar, e->X, gbar, st));
     vjp_final_kernel<double><<<grid_for((long long)N * n), 256, 0, st>>>(N, n, e->np, norm, e->rho, e->psi, gbar, ypart, Ybar);
     vjp_rho_kernel<<<1, 256, 0, st>>>(N, norm, e->N_eff, e->rho, colsum, rhobar);
     TD_CUDA(cudaGetLastError());
