@@ -138,6 +138,13 @@ int tdscha_symmetry_classes(int N_sym, int n_blocks, const int *n_deg, const dou
 int tdscha_ensemble_device_bytes(const tdscha_ensemble *ens, long long *bytes);
 
 /*
+ * The ensemble's second stream, on which the averages' F contraction may run beside Z: whether it has
+ * been made, how many events were queued for a fork and how many calls forked (graph captures count
+ * once).  For tests and tuning; no counterpart in the reference.
+ */
+int tdscha_ensemble_side_stream(const tdscha_ensemble *ens, int *made, long long *marks, long long *forks);
+
+/*
  * Symmetrised perturbed averages on host buffers: f_out (n), d2v_out (n, n) C order, exactly the
  * outputs of GetPerturbAverageSym (d2v overwritten, D4 part added when apply_d4 = 1).
  * Only the symmetric part of Y1 enters the reference's formulas; Y1 may be non-symmetric.

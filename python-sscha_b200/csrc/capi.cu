@@ -222,6 +222,14 @@ int tdscha_ensemble_device_bytes(const tdscha_ensemble *e, long long *bytes) {
     return 0;
 }
 
+int tdscha_ensemble_side_stream(const tdscha_ensemble *e, int *made, long long *marks, long long *forks) {
+    TD_CHECK(e != nullptr, TDSCHA_EINVAL, "NULL ensemble");
+    if (made) *made = e->side != nullptr;
+    if (marks) *marks = e->side_marks;
+    if (forks) *forks = e->side_forks;
+    return 0;
+}
+
 int tdscha_perturb_average_sym_device(tdscha_ensemble *e, int nb, const double *R1, const double *Y1, int apply_d4,
                                       int precision, double *f_out, double *d2v_out, void *stream) {
     clear_error();

@@ -5,6 +5,7 @@
 #include <array>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "common.cuh"
@@ -422,6 +423,7 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
 
     auto *e = new tdscha_ensemble();
     e->device = dev;
+    e->sms = prop.multiProcessorCount;
     e->n = n; e->N = N; e->N_sym = N_sym; e->n_blocks = n_blocks; e->T = T; e->dmax = dmax;
     e->P = (long long)n * (n + 1) / 2;
     e->Kp = round_up(e->P, 64);
@@ -519,13 +521,6 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
         int prc = build_pair_classes(dim, e->pairs, &pcb);
         if (prc) return fail(prc);
         e->base_bytes += pcb;
-    }
-    if (cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e->side_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e->side_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device) != cudaSuccess) {
-        set_error("creating the ensemble's second stream failed: %s", cudaGetErrorString(cudaGetLastError()));
-        return fail(TDSCHA_ECUDA);
     }
     if (cublasCreate(&e->cublas) != CUBLAS_STATUS_SUCCESS) {
         set_error("cublasCreate failed");
@@ -678,41 +673,73 @@ static int ensure_ws(tdscha_ensemble *e, size_t bytes) {
 }
 
 // The F contraction beside Z: both read the weights only, and a Z of few tiles (no symmetries, a single vector on a small
-// cell) leaves SMs idle for a chain of k-blocks as long as F's own.  begin() marks the weights' end on the caller's
-// stream; stream(): the ensemble's second stream, ordered after the mark, if Z took half the SMs or fewer, else the
-// caller's (the fork and the join cost 5 us); join() orders the caller's stream after it.  Apply on 2x2x2, us, one after
-// the other and beside: without symmetries, tf32x3, 3 vectors N = 1531 175 and 140, 32 vectors N = 4000 414 and 334; with
-// symmetries, bf16x3, N = 2000, 1 vector 176 and 153, 2 vectors (Z on most SMs) 188 and 193.
+// cell) leaves SMs idle for a chain of k-blocks as long as F's own.  Before Z's first launch planned() marks the weights' end
+// on the caller's stream if that launch takes half the SMs or fewer; stream(): the ensemble's second stream, ordered after
+// the mark, if this held for all of Z, else the caller's (the fork and the join cost 5 us); join() orders the caller's
+// stream after it, as does every other way out.  Apply on 2x2x2, us, one after the other and beside: without symmetries,
+// tf32x3, 3 vectors N = 1531 175 and 140, 32 vectors N = 4000 414 and 334; with symmetries, bf16x3, N = 2000, 1 vector
+// 176 and 153, 2 vectors (Z on most SMs) 188 and 193.
+// The second stream is made by the first fork outside a graph capture (55 us, and 75 to destroy it): most
+// ensembles (FP64, full symmetry with a few vectors) never fork.
 struct Beside {
     tdscha_ensemble *e;
     cudaStream_t st;
-    int ctas = 0;
-    bool forked = false;
-    int begin() {
-        if (!e->side) return 0;
-        TD_CUDA(cudaEventRecord(e->side_fork, st));
+    bool marked = false, forked = false;
+    std::function<int(int)> planned = [this](int ctas) {
+        const bool few = 2 * ctas <= e->sms;
+        if (!few || first) marked = few && make_side();
+        if (marked && first) {
+            TD_CUDA(cudaEventRecord(e->side_fork, st));
+            ++e->side_marks;
+        }
+        first = false;
         return 0;
-    }
+    };
+    Beside(tdscha_ensemble *e_, cudaStream_t st_) : e(e_), st(st_) {}
+    Beside(const Beside &) = delete;
+    ~Beside() { join(); }
     int stream(cudaStream_t *out) {
         *out = st;
-        if (!e->side || ctas == 0 || 2 * ctas > e->sms) return 0;
+        if (!marked) return 0;
         TD_CUDA(cudaStreamWaitEvent(e->side, e->side_fork, 0));
         forked = true;
+        ++e->side_forks;
         *out = e->side;
         return 0;
     }
     int join() {
         if (!forked) return 0;
+        forked = false;
         TD_CUDA(cudaEventRecord(e->side_join, e->side));
         TD_CUDA(cudaStreamWaitEvent(st, e->side_join, 0));
         return 0;
+    }
+
+private:
+    bool first = true;
+    bool make_side() {   // without it F stays on the caller's stream
+        if (e->side) return true;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+        cudaStream_t side = nullptr;
+        if (cudaEventCreateWithFlags(&e->side_fork, cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&e->side_join, cudaEventDisableTiming) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) == cudaSuccess) {
+            e->side = side;
+            return true;
+        }
+        cudaGetLastError();
+        for (cudaEvent_t *ev : {&e->side_fork, &e->side_join})
+            if (*ev) { cudaEventDestroy(*ev); *ev = nullptr; }
+        return false;
     }
 };
 
 // C (M x N) row-major = A (M x K) . B (N x K)^T
 static int gemm_abt(tdscha_ensemble *e, Format fmt, int nprod, const void *A_hi, const void *A_lo, long long lda, long long M,
                     const void *B_hi, const void *B_lo, long long ldb, long long N, long long K, void *Cout, long long ldc,
-                    cudaStream_t st, bool accumulate = false, int *ctas = nullptr, bool tile_sync = true) {
+                    cudaStream_t st, bool accumulate = false, const std::function<int(int)> *planned = nullptr,
+                    bool tile_sync = true) {
     if (fmt == FMT_F64) {
         const double one = 1.0, zero = accumulate ? 1.0 : 0.0;
         cublasSetStream(e->cublas, st);
@@ -739,7 +766,7 @@ static int gemm_abt(tdscha_ensemble *e, Format fmt, int nprod, const void *A_hi,
         };
         tc::GemmOperands op{fmt, nprod, off(A_hi), off(A_lo), lda, off(B_hi), off(B_lo), ldb};
         op.accumulate = accumulate || k0 > 0;
-        op.ctas = ctas;
+        op.planned = planned;
         op.tile_sync = tile_sync;
         TD_TRY(tc::gemm(op, (int)M, (int)N, (int)kc, static_cast<float *>(Cout), ldc, st, e->d_err));
     }
@@ -931,7 +958,7 @@ static int gemm_groups_f64(tdscha_ensemble *e, const std::vector<tc::GemmGroup> 
 static int gemm_groups(tdscha_ensemble *e, Format fmt, int nprod, const void *A_hi, const void *A_lo, long long a_rows,
                        long long lda, const void *B_hi, const void *B_lo, long long b_rows, long long ldb,
                        const std::vector<tc::GemmGroup> &gs, void *C, long long ldc, bool accumulate, cudaStream_t st,
-                       int drain_kb = 0, int *ctas = nullptr, bool tile_sync = true) {
+                       int drain_kb = 0, const std::function<int(int)> *planned = nullptr, bool tile_sync = true) {
     if (gs.empty()) return 0;
     if (fmt == FMT_F64)
         return gemm_groups_f64(e, gs, static_cast<const double *>(A_hi), lda, static_cast<const double *>(B_hi), ldb,
@@ -939,7 +966,7 @@ static int gemm_groups(tdscha_ensemble *e, Format fmt, int nprod, const void *A_
     tc::GemmOperands op{fmt, nprod, A_hi, A_lo, lda, B_hi, B_lo, ldb};
     op.accumulate = accumulate;
     op.drain_kb = drain_kb;
-    op.ctas = ctas;
+    op.planned = planned;
     op.tile_sync = tile_sync;
     return tc::gemm_grouped(op, a_rows, lda, b_rows, ldb, gs.data(), (int)gs.size(), static_cast<float *>(C), ldc, st, e->d_err);
 }
@@ -1160,13 +1187,12 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
                     TD_TRY(freq_weights<float>(ft, (const float *)H, (const float *)Ch, L.ld1, e->rho + c0, Ncur, NR, N2pc,
                                                apply_d4, fmt, Cw_hi, Cw_lo, AB_hi, AB_lo, st));
             }
-            Beside f{e, st};
+            Beside f(e, st);
             cudaStream_t fs = st;
-            TD_TRY(f.begin());
             {
                 StageScope sc(e, ST_GEMM_Z, st);
                 TD_TRY(gemm_groups(e, fmt, nprod, Cw_hi, Cw_lo, (long long)nC * 2 * NR, N2pc, co.VT_hi, co.VT_lo, ft.Kq, N2pc,
-                                   gz, O, ft.Kq, acc, st, 0, &f.ctas));
+                                   gz, O, ft.Kq, acc, st, 0, &f.planned));
             }
             TD_TRY(f.stream(&fs));
             {
@@ -1389,13 +1415,12 @@ int perturb_average_device(tdscha_ensemble *e, int nb, const double *R1, const d
                         Cw_lo, AB_hi, AB_lo);
                 TD_CUDA(cudaGetLastError());
             }
-            Beside fb{e, st};
+            Beside fb(e, st);
             cudaStream_t fs = st;
-            TD_TRY(fb.begin());
             // GEMM2: Z (+)= Cw . VT^T          (M x P, K = N2pc)
             {
                 StageScope sc(e, ST_GEMM_Z, st);
-                TD_TRY(gemm_abt(e, fmt, nprod, Cw_hi, Cw_lo, N2pc, M, co.VT_hi, co.VT_lo, N2pc, e->P, N2pc, Z, L.ldz, st, acc, &fb.ctas));
+                TD_TRY(gemm_abt(e, fmt, nprod, Cw_hi, Cw_lo, N2pc, M, co.VT_hi, co.VT_lo, N2pc, e->P, N2pc, Z, L.ldz, st, acc, &fb.planned));
             }
             TD_TRY(fb.stream(&fs));
             // F (+)= AB . YXt^T                (M x n, K = N2pc)

@@ -103,6 +103,7 @@ struct tdscha_ensemble {
     void *dg_part = nullptr;                       // scratch of the split FP64 contractions (dgemm.cuh), built by the first
     cudaStream_t side = nullptr;                   // F's contraction beside Z's
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    long long side_marks = 0, side_forks = 0;
     int sms = 0;
     tdscha::AvgPlan plan;                          // chunking plan of the last averages call
     double *YX = nullptr;                          // [Y; X~] (2N x np), FP64, built by the first VJP

@@ -1252,6 +1252,7 @@ static int launch_tuned(const GemmOperands &op, const WeightsOut *wo, const Prob
         }
         TilePlan pl;
         const TileShape sh = choose_shape(pb, g0, g1, key, KBlock<TF32, 128>::ELEMS, NPROD, drain, sms, stall != 0, &pl);
+        if (op.planned) TD_TRY((*op.planned)((int)std::min<long long>(pl.tiles, sms)));
         Prepared cfg;
         TD_TRY((prepare<TF32, NPROD>(op, wo, pb, g0, g1, sh, pl, D, ldd, st, err, counter, stall, sms, &cfg)));
         int gp = cfg.num_p;
@@ -1261,7 +1262,6 @@ static int launch_tuned(const GemmOperands &op, const WeightsOut *wo, const Prob
         if (!stall) TD_TRY(choose_order(key, cfg, sms, st, !op.accumulate && !capturing, &gp));
         cfg.launch(gp);
         TD_CUDA(cudaGetLastError());
-        if (op.ctas) *op.ctas = std::max(*op.ctas, (int)std::min<long long>(pl.tiles, sms));
     }
     return 0;
 }

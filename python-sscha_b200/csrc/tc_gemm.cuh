@@ -1,6 +1,7 @@
 // tc_gemm.cuh -- interface of the tcgen05 contraction kernel (tc_gemm.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <functional>
 #include <vector>
 #include "common.cuh"
 
@@ -20,7 +21,7 @@ struct GemmOperands {
     int drain_kb = 0;   // k-blocks per TMEM chunk drained to fp32 registers (0 = library default)
     bool accumulate = false;   // D += A . B^T instead of D = A . B^T
     bool tile_sync = true;     // co-resident tiles may wait for one another (bounded) to share operand slices
-    int *ctas = nullptr;       // out: most CTAs of one of the launches
+    const std::function<int(int)> *planned = nullptr;   // called before each launch with its CTAs
 };
 
 // K must be a multiple of 64 (bf16) or 32 (tf32); operands must be readable up to K columns.

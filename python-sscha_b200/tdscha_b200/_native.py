@@ -93,6 +93,8 @@ def load():
     lib.tdscha_debug_stall_next_contraction.argtypes = []
     lib.tdscha_set_error_check.argtypes = [ctypes.c_int]
     lib.tdscha_check_errors.argtypes = [vp, vp]
+    lib.tdscha_ensemble_side_stream.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]
+    lib.tdscha_ensemble_side_stream.restype = ctypes.c_int
     lib.tdscha_set_profiling.argtypes = [vp, ctypes.c_int]
     lib.tdscha_read_profile.argtypes = [vp, dp, ctypes.POINTER(ctypes.c_longlong), ctypes.c_int]
     for name in ("tdscha_perturb_average_vjp_precision_device", "tdscha_set_wait_budget", "tdscha_debug_stall_next_contraction", "tdscha_apply_L1_static_device", "tdscha_apply_static_L_device", "tdscha_lanczos_run_device", "tdscha_lanczos_step_device_noalloc", "tdscha_apply_prologue_device", "tdscha_apply_epilogue_device", "tdscha_set_profiling", "tdscha_read_profile", "tdscha_tc_contract", "tdscha_ensemble_create", "tdscha_ensemble_destroy", "tdscha_ensemble_info",
@@ -163,6 +165,12 @@ class DeviceEnsemble:
         b = ctypes.c_longlong()
         check(self._lib.tdscha_ensemble_device_bytes(self.handle, ctypes.byref(b)))
         return b.value
+
+    def side_stream(self):
+        """dict(made, marks, forks) of the second stream of the averages (tdscha_ensemble_side_stream)."""
+        made, marks, forks = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_longlong()
+        check(self._lib.tdscha_ensemble_side_stream(self.handle, ctypes.byref(made), ctypes.byref(marks), ctypes.byref(forks)))
+        return dict(made=bool(made.value), marks=marks.value, forks=forks.value)
 
     def cosets(self):
         """The factorised symmetry path: dict(rotated, n_cosets, coset_size, offpattern)
