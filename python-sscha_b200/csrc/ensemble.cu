@@ -686,7 +686,7 @@ struct Beside {
     cudaStream_t st;
     bool marked = false, forked = false;
     std::function<int(int)> planned = [this](int ctas) {
-        const bool few = 2 * ctas <= e->sms;
+        const bool few = 2 * ctas <= e->sms && !e->prof.enabled;   // a profile is of the caller's stream, stage after stage
         if (!few || first) marked = few && make_side();
         if (marked && first) {
             TD_CUDA(cudaEventRecord(e->side_fork, st));

@@ -38,3 +38,22 @@ def test_made_by_the_first_fork(cuda, sym, nb, precision, forks):
         _call(cuda, ens, v, precision)
         assert ens.side_stream() == dict(made=forks > 0, marks=call * forks, forks=call * forks)
     ens.close()
+
+
+# a profile holds events of the launching stream only, so F stays there while it is taken; the contraction is the
+# same launch on either stream, so the bits are the same
+@pytest.mark.parametrize("sym,nb,precision", [(False, 3, "tf32x3"), (False, 32, "bf16x3"), (True, 1, "bf16x3")])
+def test_profiled_calls_stay_on_the_launching_stream(cuda, sym, nb, precision):
+    ens = _ensemble(sym)
+    v = _vectors(cuda, ens, nb)
+    f0, d0 = _call(cuda, ens, v, precision)
+    assert ens.side_stream()["forks"] == 1
+    ens.set_profiling(True)
+    f1, d1 = _call(cuda, ens, v, precision)
+    assert ens.side_stream()["forks"] == 1
+    assert ens.read_profile()["gemm_f"][0] > 0.0
+    ens.set_profiling(False)
+    f2, d2 = _call(cuda, ens, v, precision)
+    assert ens.side_stream()["forks"] == 2
+    assert cuda.equal(f1, f0) and cuda.equal(d1, d0) and cuda.equal(f2, f0) and cuda.equal(d2, d0)
+    ens.close()
