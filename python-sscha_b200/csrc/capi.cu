@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <vector>
 
@@ -56,18 +57,38 @@ static int scratch_get(int slot, size_t bytes, cudaStream_t st, void **out) {
 // Per-call reading of the error word (tdscha_set_error_check); off: tdscha_check_errors reads it.
 static std::atomic<int> g_check_per_call{1};
 
-// The word lands in page-locked memory, one word per host thread (kept for the thread's life): a copy
-// to pageable memory goes through the driver's staging buffer.
+// The word lands in page-locked memory (a copy to pageable memory goes through the driver's staging buffer), one word per
+// host thread.  A thread that ends hands its word to the next one: freeing it would end a graph capture of any other thread
+// with an error, and wait for the device.  There are never more words than threads that lived at the same time.
 struct PinnedWord {
     unsigned *p = nullptr;
     ~PinnedWord() {
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        std::lock_guard<std::mutex> lock(mutex());
+        idle().push_back(p);
     }
+    int get() {
+        if (p) return 0;
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            if (!idle().empty()) {
+                p = idle().back();
+                idle().pop_back();
+                return 0;
+            }
+        }
+        TD_CUDA(cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable));
+        return 0;
+    }
+
+private:   // never destroyed: threads may outlive the library's statics
+    static std::mutex &mutex() { static auto *m = new std::mutex; return *m; }
+    static std::vector<unsigned *> &idle() { static auto *v = new std::vector<unsigned *>; return *v; }
 };
 static thread_local PinnedWord g_err_word;
 
 static int read_err_word(tdscha_ensemble *e, cudaStream_t st) {
-    if (!g_err_word.p) TD_CUDA(cudaHostAlloc(&g_err_word.p, sizeof(unsigned), cudaHostAllocPortable));
+    TD_TRY(g_err_word.get());
     TD_CUDA(cudaMemcpyAsync(g_err_word.p, e->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     TD_CUDA(cudaStreamSynchronize(st));
     const unsigned h = *g_err_word.p;
