@@ -10,7 +10,6 @@
 
 #include "apply.cuh"
 #include "common.cuh"
-#include "dgemm.cuh"
 #include "ensemble.cuh"
 #include "freq.cuh"
 #include "modes.cuh"
@@ -234,7 +233,7 @@ int tdscha_symmetry_cosets(int N_sym, int n_blocks, const int *n_deg, const doub
 
 int tdscha_ensemble_device_bytes(const tdscha_ensemble *e, long long *bytes) {
     TD_CHECK(e != nullptr && bytes != nullptr, TDSCHA_EINVAL, "NULL argument");
-    size_t b = e->base_bytes + e->ws.bytes + (e->dg_part ? tdscha::dgemm_part_bytes() : 0);
+    size_t b = e->base_bytes + e->ws.bytes;
     for (const auto &o : e->ops) b += o.bytes;
     for (const auto &o : e->fops) b += o.bytes;
     for (const auto &o : e->fhalf) b += o.bytes;

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(THREADS) dgemm_grouped_kernel(const double *__
 
 template <int BM, int BN>
 int launch(const double *A, long long lda, const double *B, long long ldb, const tc::GemmGroup *gs, int n, double *C, long long ldc,
-           bool accumulate, void *part, cudaStream_t st) {
+           bool accumulate, double *part, unsigned *count, cudaStream_t st) {
     DTable t{};
     t.n = n;
     int tiles = 0, kmax = 0;
@@ -166,29 +166,26 @@ int launch(const double *A, long long lda, const double *B, long long ldb, const
         tiles += d.tiles_m * ceil_div(d.N, BN);
         kmax = std::max(kmax, d.K);
     }
-    // slices of K: until the launch has four CTAs per SM, none shorter than 16 k-blocks
     // Slices of K (8 k-blocks at least): the machine takes ceil(CTAs / 148) rounds of one slice each, to which a CTA
     // adds about 14 k-blocks of start, write-out and adding up, and the last CTA the latency of its own slice.  Against
     // four CTAs per SM whatever the shape: F of 32 vectors on 2x2x2 276 -> 228 us, Z of 8 vectors 168 -> 130.
     t.slices = 1;
     double best = 1e300;
-    for (int s = 1; s == 1 || (part && s * tiles <= MAX_CTAS && s <= kmax / BK / 8); ++s) {
+    for (int s = 1; s == 1 || (s * tiles <= MAX_CTAS && s <= kmax / BK / 8); ++s) {
         const double kb = (double)kmax / BK / s, cost = ceil_div(tiles * s, 148) * (kb + 14.0) + 2.0 * kb;
         if (cost < best) { best = cost; t.slices = s; }
     }
-    unsigned *count = static_cast<unsigned *>(part);
     constexpr int smem = STAGES * (BM + BN) * LDS * (int)sizeof(double);
     TD_TRY((allow_smem<dgemm_grouped_kernel<BM, BN>>(smem)));
     dgemm_grouped_kernel<BM, BN><<<dim3((unsigned)tiles, (unsigned)t.slices), THREADS, smem, st>>>(A, lda, B, ldb, C, ldc, t,
-                                                                                            reinterpret_cast<double *>(count + MAX_CTAS), count,
-                                                                                            accumulate ? 1 : 0);
+                                                                                                   part, count, accumulate ? 1 : 0);
     TD_CUDA(cudaGetLastError());
     return 0;
 }
 
 }  // namespace
 
-size_t dgemm_part_bytes() { return DGEMM_COUNT_BYTES + (size_t)MAX_CTAS * 64 * 64 * sizeof(double); }
+size_t dgemm_part_bytes() { return (size_t)MAX_CTAS * 64 * 64 * sizeof(double); }
 
 bool dgemm_fits(const double *A, long long lda, const double *B, long long ldb, const std::vector<tc::GemmGroup> &gs) {
     bool ok = lda % 2 == 0 && ldb % 2 == 0 && (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) % 16 == 0;
@@ -197,7 +194,7 @@ bool dgemm_fits(const double *A, long long lda, const double *B, long long ldb, 
 }
 
 int dgemm_grouped(const double *A, long long lda, const double *B, long long ldb, const std::vector<tc::GemmGroup> &gs, double *C,
-                  long long ldc, bool accumulate, void *part, cudaStream_t st) {
+                  long long ldc, bool accumulate, double *part, unsigned *count, cudaStream_t st) {
     // 64-row tiles move half the operand bytes per product of 32-row ones (4 % faster where neither pads: [a|b] of 2 vectors
     // on 3x3x3, N = 20000, 6.25 and 6.54 ms); 32 where 64 would compute 1.1 times the rows or more (2 vectors on 2x2x2:
     // Z 46 us, with 64 rows 56).
@@ -215,7 +212,7 @@ int dgemm_grouped(const double *A, long long lda, const double *B, long long ldb
     const auto run = nmax <= 16 ? (m64 ? launch<64, 16> : launch<32, 16>) : (m64 ? launch<64, 64> : launch<32, 64>);
     for (size_t i = 0; i < gs.size(); i += MAX_G) {
         const int n = (int)std::min<size_t>(MAX_G, gs.size() - i);
-        TD_TRY(run(A, lda, B, ldb, gs.data() + i, n, C, ldc, accumulate, part, st));
+        TD_TRY(run(A, lda, B, ldb, gs.data() + i, n, C, ldc, accumulate, part, count, st));
     }
     return 0;
 }

@@ -247,6 +247,8 @@ static int grid_for(long long total, int threads = 256) {
     return (int)std::min<long long>(std::max<long long>(g, 1), 148LL * 32);
 }
 
+constexpr size_t ERR_BYTES = 256;   // the error word, in front of the counters of the split FP64 contractions
+
 static int dev_alloc(void **p, size_t bytes, size_t *acc) {
     TD_CUDA(cudaMalloc(p, bytes));
     if (acc) *acc += bytes;
@@ -468,7 +470,7 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
         (rc = dev_alloc((void **)&e->d_pair_mu, e->P * sizeof(int), &acc)) ||
         (rc = dev_alloc((void **)&e->d_pair_nu, e->P * sizeof(int), &acc)) ||
         (rc = dev_alloc((void **)&e->wfac, e->P * sizeof(float), &acc)) ||
-        (rc = dev_alloc((void **)&e->d_err, sizeof(unsigned), &acc)))
+        (rc = dev_alloc((void **)&e->d_err, ERR_BYTES + DGEMM_COUNT_BYTES, &acc)))
         return fail(rc);
     e->base_bytes = acc;
     std::vector<int> pmu(e->P), pnu(e->P);
@@ -498,7 +500,8 @@ int ensemble_create(const double *X, const double *Y, const double *w, const dou
     TD_UP(e->d_pair_mu, pmu.data(), e->P * sizeof(int));
     TD_UP(e->d_pair_nu, pnu.data(), e->P * sizeof(int));
 #undef TD_UP
-    if (cudaMemset(e->d_err, 0, sizeof(unsigned)) != cudaSuccess) return fail(TDSCHA_ECUDA);
+    if (cudaMemset(e->d_err, 0, ERR_BYTES + DGEMM_COUNT_BYTES) != cudaSuccess) return fail(TDSCHA_ECUDA);
+    e->dg_count = e->d_err + ERR_BYTES / sizeof(unsigned);
     if (cosets_enabled()) {
         const int crc = setup_cosets(e, dim, sym_blocks);
         if (crc) return fail(crc);
@@ -547,7 +550,7 @@ int ensemble_destroy(tdscha_ensemble *e) {
     if (e->side_fork) cudaEventDestroy(e->side_fork);
     if (e->side_join) cudaEventDestroy(e->side_join);
     void *ps[] = {e->X, e->Y, e->G, e->Xt, e->rho, e->w, e->ups, e->psi, e->sym, e->symP, e->symPT, e->d_offP, e->d_blk_start, e->d_blk_dim,
-                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->dg_part, e->ws.base,
+                  e->d_blk_sym_off, e->d_blocks_ids, e->d_bp_b, e->d_bp_c, e->d_pair_mu, e->d_pair_nu, e->d_err, e->wfac, e->ws.base,
                   e->vjp_ws.base, e->YX, e->chunk_ops.base, e->XGT, e->d_static_lam, e->Rrow, e->d_grp, e->rot_ws.base};
     for (void *p : ps)
         if (p) cudaFree(p);
@@ -877,7 +880,7 @@ static int ensure_freq_operands(tdscha_ensemble *e, Format fmt, bool lo, cudaStr
 }
 
 struct FreqWs {
-    size_t U, r1, Lab_hi, Lab_lo, Lcd_hi, Lcd_lo, H, Ch, Cw_hi, Cw_lo, AB_hi, AB_lo, O, OF, partD, partF, Ysr, R1r;
+    size_t U, r1, Lab_hi, Lab_lo, Lcd_hi, Lcd_lo, H, Ch, Cw_hi, Cw_lo, AB_hi, AB_lo, O, OF, partD, partF, Ysr, R1r, part;
     size_t total;
     long long ld1, ldz, ldf, N2pc;
 };
@@ -912,25 +915,9 @@ static FreqWs freq_ws_layout(const tdscha_ensemble *e, int nb, int ncj, int nf_t
     L.partF = take((size_t)nb * nf_total * e->n * 8);
     L.Ysr = take((size_t)nb * e->n * e->n * 8);
     L.R1r = take((size_t)nb * e->n * 8);
+    L.part = fmt == FMT_F64 ? take(dgemm_part_bytes()) : 0;
     L.total = off;
     return L;
-}
-
-// Scratch of the grouped FP64 kernel, once per ensemble and never moved (captured graphs hold its address).  Without
-// it (first call under capture, no memory left) the contractions are not split.
-static int ensure_dg_part(tdscha_ensemble *e, cudaStream_t st) {
-    if (e->dg_part) return 0;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    TD_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return 0;
-    void *p = nullptr;
-    if (cudaMalloc(&p, dgemm_part_bytes()) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    e->dg_part = p;
-    TD_CUDA(cudaMemsetAsync(p, 0, DGEMM_COUNT_BYTES, st));
-    return 0;
 }
 
 // C (row-major) (+)= A . B^T for every group, FP64.  Groups of up to 2 GF on average go through the grouped kernel of
@@ -938,13 +925,11 @@ static int ensure_dg_part(tdscha_ensemble *e, cudaStream_t st) {
 // and grouped kernel, us: 0.66 GF a class 770 and 683, 2.6 GF 2588 and 2489 (Z: 2510 and 2601), 6.6 GF 5736 and 6527).
 constexpr double DG_FLOPS = 2e9;
 static int gemm_groups_f64(tdscha_ensemble *e, const std::vector<tc::GemmGroup> &gs, const double *A, long long lda,
-                           const double *B, long long ldb, double *C, long long ldc, bool accumulate, cudaStream_t st) {
+                           const double *B, long long ldb, double *C, long long ldc, bool accumulate, double *part, cudaStream_t st) {
     double flops = 0.0;
     for (const auto &g : gs) flops += 2.0 * g.M * g.N * g.K;
-    if (flops <= DG_FLOPS * gs.size() && dgemm_fits(A, lda, B, ldb, gs)) {
-        TD_TRY(ensure_dg_part(e, st));
-        return dgemm_grouped(A, lda, B, ldb, gs, C, ldc, accumulate, e->dg_part, st);
-    }
+    if (flops <= DG_FLOPS * gs.size() && dgemm_fits(A, lda, B, ldb, gs))
+        return dgemm_grouped(A, lda, B, ldb, gs, C, ldc, accumulate, part, e->dg_count, st);
     const double one = 1.0, beta = accumulate ? 1.0 : 0.0;
     cublasSetStream(e->cublas, st);
     for (const auto &g : gs) {
@@ -957,12 +942,12 @@ static int gemm_groups_f64(tdscha_ensemble *e, const std::vector<tc::GemmGroup> 
 
 static int gemm_groups(tdscha_ensemble *e, Format fmt, int nprod, const void *A_hi, const void *A_lo, long long a_rows,
                        long long lda, const void *B_hi, const void *B_lo, long long b_rows, long long ldb,
-                       const std::vector<tc::GemmGroup> &gs, void *C, long long ldc, bool accumulate, cudaStream_t st,
+                       const std::vector<tc::GemmGroup> &gs, void *C, long long ldc, bool accumulate, double *part, cudaStream_t st,
                        int drain_kb = 0, const std::function<int(int)> *planned = nullptr, bool tile_sync = true) {
     if (gs.empty()) return 0;
     if (fmt == FMT_F64)
         return gemm_groups_f64(e, gs, static_cast<const double *>(A_hi), lda, static_cast<const double *>(B_hi), ldb,
-                               static_cast<double *>(C), ldc, accumulate, st);
+                               static_cast<double *>(C), ldc, accumulate, part, st);
     tc::GemmOperands op{fmt, nprod, A_hi, A_lo, lda, B_hi, B_lo, ldb};
     op.accumulate = accumulate;
     op.drain_kb = drain_kb;
@@ -1087,6 +1072,7 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
     double *Ysr = static_cast<double *>(at(L.Ysr)), *R1r = static_cast<double *>(at(L.R1r));
     const bool f64 = fmt == FMT_F64;
     const size_t as = f64 ? 8 : 4;
+    double *part = f64 ? static_cast<double *>(at(L.part)) : nullptr;
     {
         StageScope sc(e, ST_OTHER, st, 1);
         TD_TRY(rotate_in(e->rot, nb, Ys, R1, Ysr, R1r, st));
@@ -1172,12 +1158,12 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
                 {
                     StageScope sc(e, ST_GEMM_AB, st);
                     TD_TRY(gemm_groups(e, fmt, nprod, Lab_hi, Lab_lo, 2LL * NR, ft.Kq, co.V_hi, co.V_lo, brows, ft.Kq, gab, H, L.ld1,
-                                       false, st, freq_ab_drain()));
+                                       false, part, st, freq_ab_drain()));
                 }
                 {
                     StageScope sc(e, ST_GEMM_CD, st);
                     TD_TRY(gemm_groups(e, fmt, nprod, Lcd_hi, Lcd_lo, 2LL * NR, Kmq1, co.XG_hi, co.XG_lo, brows, Kmq1, gcd, Ch, L.ld1,
-                                       false, st));
+                                       false, part, st));
                 }
                 StageScope sc(e, ST_WEIGHTS, st);
                 if (f64)
@@ -1192,13 +1178,13 @@ static int perturb_average_freq(tdscha_ensemble *e, int nb, const double *R1, co
             {
                 StageScope sc(e, ST_GEMM_Z, st);
                 TD_TRY(gemm_groups(e, fmt, nprod, Cw_hi, Cw_lo, (long long)nC * 2 * NR, N2pc, co.VT_hi, co.VT_lo, ft.Kq, N2pc,
-                                   gz, O, ft.Kq, acc, st, 0, &f.planned));
+                                   gz, O, ft.Kq, acc, part, st, 0, &f.planned));
             }
             TD_TRY(f.stream(&fs));
             {
                 StageScope sc(e, ST_GEMM_F, fs);
                 TD_TRY(gemm_groups(e, fmt, nprod, AB_hi, AB_lo, (long long)nC * 2 * NR, N2pc, co.YX_hi, co.YX_lo, Kmq1, N2pc,
-                                   gf, OF, Kmq1, acc, fs, 0, nullptr, fs == st));
+                                   gf, OF, Kmq1, acc, part, fs, 0, nullptr, fs == st));
             }
             TD_TRY(f.join());
         }
@@ -1879,7 +1865,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     const FreqOps &co = e->fops[fmt];
     // workspace: fixed part, then per coset (NR = nb * cosets of the chunk, NRp = NR rounded to 64)
     const size_t fixed = as * ((size_t)N * Kq + 2 * (size_t)N * Kmq1 + (size_t)N * e->Kp + 2 * (size_t)N * e->np) +
-                         8 * ((size_t)N * (1 + COLSUM_SLICES) + (size_t)nb * n + (size_t)nb * n * n) + 33 * 256;
+                         8 * ((size_t)N * (1 + COLSUM_SLICES) + (size_t)nb * n + (size_t)nb * n * n) + (f64 ? dgemm_part_bytes() : 0) + 34 * 256;
     auto per_chunk = [&](int ncj) {
         const size_t NR = (size_t)nb * ncj, NRp = round_up(NR, 64), rows = (size_t)nC * 2 * NR;
         size_t b = 2 * as * (NR * e->Kp + NR * e->np);                      // U, r1, Q, phi
@@ -1913,6 +1899,7 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
     double *colsum = static_cast<double *>(take(8 * (size_t)N));
     double *colpart = static_cast<double *>(take(8 * (size_t)N * COLSUM_SLICES));
     double *Rq = static_cast<double *>(take(8 * (size_t)nb * n)), *Dq = static_cast<double *>(take(8 * (size_t)nb * n * n));
+    double *part = f64 ? static_cast<double *>(take(dgemm_part_bytes())) : nullptr;
     void *U = take(as * NRmax * e->Kp), *r1 = take(as * NRmax * e->np), *Q = take(as * NRmax * e->Kp), *phi = take(as * NRmax * e->np);
     auto pair_of = [&](size_t count) { void *h = take(count * es); void *l = lo ? take(count * es) : nullptr; return std::make_pair(h, l); };
     auto Lab = pair_of(2 * NRmax * Kq), LQ = pair_of(2 * NRmax * Kq), Lcd = pair_of(2 * NRmax * Kmq1), Lph = pair_of(2 * NRmax * Kmq1);
@@ -1967,11 +1954,11 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
                 TD_CUDA(cudaMemsetAsync(static_cast<uint8_t *>(Cp) + hrow * ld1 * as, 0, (size_t)2 * NR * ld1 * as, st));
             }
         }
-        TD_TRY(gemm_groups(e, fmt, nprod, Lab.first, Lab.second, 2LL * NR, Kq, co.V_hi, co.V_lo, e->N2, Kq, gab, H, ld1, false, st));
-        TD_TRY(gemm_groups(e, fmt, nprod, LQ.first, LQ.second, 2LL * NR, Kq, co.V_hi, co.V_lo, e->N2, Kq, gab, HQ, ld1, false, st));
-        TD_TRY(gemm_groups(e, fmt, nprod, Lcd.first, Lcd.second, 2LL * NR, Kmq1, co.XG_hi, co.XG_lo, e->N2, Kmq1, gcd, Ch, ld1, false, st));
+        TD_TRY(gemm_groups(e, fmt, nprod, Lab.first, Lab.second, 2LL * NR, Kq, co.V_hi, co.V_lo, e->N2, Kq, gab, H, ld1, false, part, st));
+        TD_TRY(gemm_groups(e, fmt, nprod, LQ.first, LQ.second, 2LL * NR, Kq, co.V_hi, co.V_lo, e->N2, Kq, gab, HQ, ld1, false, part, st));
+        TD_TRY(gemm_groups(e, fmt, nprod, Lcd.first, Lcd.second, 2LL * NR, Kmq1, co.XG_hi, co.XG_lo, e->N2, Kmq1, gcd, Ch, ld1, false, part, st));
         TD_TRY(gemm_groups(e, fmt, nprod, Lph.first, Lph.second, 2LL * NR, Kmq1, e->fyx_hi[fmt], lo ? e->fyx_lo[fmt] : nullptr,
-                           e->N2, Kmq1, gcd, Cp, ld1, false, st));
+                           e->N2, Kmq1, gcd, Cp, ld1, false, part, st));
         // coefficients and the rho pairing
         void *Kh[4] = {Ks[0].first, Ks[1].first, Ks[2].first, Ks[3].first};
         void *Kl[4] = {Ks[0].second, Ks[1].second, Ks[2].second, Ks[3].second};
@@ -2030,10 +2017,10 @@ static int perturb_average_vjp_freq(tdscha_ensemble *e, int nb, const double *R1
                 gp.push_back({N, ft.pcol_cnt[g], Kg, 0, a_k, ft.pcol_off[g], 0, (long long)ft.pcol_off[g]});
                 if (ft.mcol_cnt[g] > 0) gm.push_back({N, ft.mcol_cnt[g], Kg, 0, a_k, ft.mcol_off[g], 0, (long long)ft.mcol_off[g]});
             }
-            TD_TRY(gemm_groups(e, fmt, nprod, Kh[0], Kl[0], N, RT, LabT.first, LabT.second, Kq, 2LL * NRp, gp, VbarQ, Kq, !first, st));
-            TD_TRY(gemm_groups(e, fmt, nprod, Kh[1], Kl[1], N, RT, LQT.first, LQT.second, Kq, 2LL * NRp, gp, VbarQ, Kq, true, st));
-            TD_TRY(gemm_groups(e, fmt, nprod, Kh[2], Kl[2], N, RT, LcdT.first, LcdT.second, Kmq1, 2LL * NRp, gm, GQ, Kmq1, !first, st));
-            TD_TRY(gemm_groups(e, fmt, nprod, Kh[3], Kl[3], N, RT, LphT.first, LphT.second, Kmq1, 2LL * NRp, gm, YQ, Kmq1, !first, st));
+            TD_TRY(gemm_groups(e, fmt, nprod, Kh[0], Kl[0], N, RT, LabT.first, LabT.second, Kq, 2LL * NRp, gp, VbarQ, Kq, !first, part, st));
+            TD_TRY(gemm_groups(e, fmt, nprod, Kh[1], Kl[1], N, RT, LQT.first, LQT.second, Kq, 2LL * NRp, gp, VbarQ, Kq, true, part, st));
+            TD_TRY(gemm_groups(e, fmt, nprod, Kh[2], Kl[2], N, RT, LcdT.first, LcdT.second, Kmq1, 2LL * NRp, gm, GQ, Kmq1, !first, part, st));
+            TD_TRY(gemm_groups(e, fmt, nprod, Kh[3], Kl[3], N, RT, LphT.first, LphT.second, Kmq1, 2LL * NRp, gm, YQ, Kmq1, !first, part, st));
         }
         first = false;
     }

@@ -100,7 +100,7 @@ struct tdscha_ensemble {
     tdscha::Workspace ws;
     tdscha::Workspace vjp_ws;                      // workspace of the averages' VJP
     tdscha::Workspace chunk_ops;                   // operands of one configuration chunk (large ensembles)
-    void *dg_part = nullptr;                       // scratch of the split FP64 contractions (dgemm.cuh), built by the first
+    unsigned *dg_count = nullptr;                  // counters of the split FP64 contractions (dgemm.cuh), in d_err's allocation
     cudaStream_t side = nullptr;                   // F's contraction beside Z's
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
     long long side_marks = 0, side_forks = 0;
