@@ -443,8 +443,9 @@ struct CFParams {
 // scaled by a power of two every CF_GROUP steps.  Im(P / Q) would be the difference of two products that grow more
 // alike with every step (a spectral function far below the real part lost three digits in 1500 steps), so
 // D = Im(P conj Q) is carried beside them, D <- bc D - Im(d) |Q|^2, a sum of one sign where bc > 0, and Im(g) = D / |Q|^2.
-// A denominator of zero, or a |Q|^2 that leaves the range of a double within a group, goes through the division per step
-// as written (same infinities and NaN).
+// The coefficients are taken in units of a power of two near a[0], so that |Q|^2 stays in the range of a double whatever unit
+// they come in.  A denominator of zero, or a |Q|^2 that leaves that range within a group all the same, goes through the
+// division per step as written (same infinities and NaN).
 // 100 steps, 500 frequencies: 18.3 -> 8 us (with a group of 4 steps 9).
 constexpr int CF_THREADS = 32, CF_CHUNK = 256, CF_GROUP = 8;
 
@@ -481,8 +482,10 @@ __global__ void __launch_bounds__(CF_THREADS) cf_kernel(CFParams prm, const doub
         const double A = a[prm.n_iter - 1] * prm.sign - prm.sign * prm.shift;
         g = cuCdiv(make_cuDoubleComplex(1.0, 0.0), make_cuDoubleComplex(A + wsgn * w * w, 2 * w * prm.smearing));
     }
-    const double ww = wsgn * w * w, di = 2 * w * prm.smearing;
-    double Pr = cuCreal(g), Pi = cuCimag(g), Qr = 1.0, Qi = 0.0, D = Pi, QQ = 1.0;   // QQ = |Q|^2
+    const int e0 = (__double2hiint(a[0]) >> 20) & 0x7ff, ks = e0 > 523 && e0 < 1523 ? e0 - 1023 : 0;
+    const double unit = __hiloint2double((1023 + ks) << 20, 0), inv = __hiloint2double((1023 - ks) << 20, 0);   // 2^ks and its inverse
+    const double ww = wsgn * w * w * inv, di = 2 * w * prm.smearing * inv;
+    double Pr = cuCreal(g) * unit, Pi = cuCimag(g) * unit, Qr = 1.0, Qi = 0.0, D = Pi, QQ = 1.0;   // QQ = |Q|^2
     bool plain = prm.n_iter < 2;   // nothing to advance: g stands
     for (int top = prm.n_iter - 2; top >= 0; top -= CF_CHUNK) {   // steps top, top - 1, ...
         const int m = min(top + 1, CF_CHUNK);
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(CF_THREADS) cf_kernel(CFParams prm, const doub
         for (int j = threadIdx.x; j < m; j += CF_THREADS) {
             const int i = top - j;
             const double B = b[i] * prm.sign, C = nonsym ? c[i] * prm.sign : B;
-            co[j] = make_double2(a[i] * prm.sign - prm.sign * prm.shift, B * C);
+            co[j] = make_double2((a[i] * prm.sign - prm.sign * prm.shift) * inv, B * inv * (C * inv));
         }
         __syncthreads();
         for (int j0 = 0; j0 < m; j0 += CF_GROUP) {
@@ -533,7 +536,7 @@ __global__ void __launch_bounds__(CF_THREADS) cf_kernel(CFParams prm, const doub
             g = cuCdiv(make_cuDoubleComplex(1.0, 0.0), den);
         }
     } else {
-        g = make_cuDoubleComplex(cuCreal(cuCdiv(make_cuDoubleComplex(Pr, Pi), make_cuDoubleComplex(Qr, Qi))), D / QQ);
+        g = make_cuDoubleComplex(cuCreal(cuCdiv(make_cuDoubleComplex(Pr, Pi), make_cuDoubleComplex(Qr, Qi))) * inv, D / QQ * inv);
     }
     double re = cuCreal(g), im = cuCimag(g);
     if (prm.use_wigner) re = -re;

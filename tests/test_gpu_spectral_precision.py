@@ -20,7 +20,7 @@ def _fraction(a, b, c, w, eta, wigner):
 # 1.5 times their number, 6 ulp; 16 ulp allowed.
 @pytest.mark.parametrize("n_iter", [2, 9, 100, 300, 1500])
 @pytest.mark.parametrize("eta", [1e-2, 1e-4, 1e-9])
-@pytest.mark.parametrize("scale", [1e-6, 1.0])
+@pytest.mark.parametrize("scale", [1e-20, 1e-6, 1.0, 1e26])
 @pytest.mark.parametrize("wigner", [False, True])
 def test_imaginary_part_outside_the_band(cuda, n_iter, eta, scale, wigner):
     torch = cuda
