@@ -301,7 +301,8 @@ int tdscha_continued_fraction_device(int n_iter, const double *a, const double *
  * milliseconds and the launch counts of the n_stages stages (0 transform, 1 contraction [a|b],
  * 2 contraction [c|d], 3 weights, 4 contraction Z, 5 contraction F, 6 fold, 7 other, 8 the
  * operand rebuilds of configuration-chunked ensembles) since the last read, and resets them.
- * Launch counts are kept even with profiling disabled.
+ * Launch counts are kept even with profiling disabled.  Stages never overlap: while profiling is
+ * enabled the F contraction does not run on the ensemble's second stream.
  */
 int tdscha_set_profiling(tdscha_ensemble *ens, int enable);
 int tdscha_read_profile(tdscha_ensemble *ens, double *ms, long long *launches, int n_stages);
@@ -348,7 +349,8 @@ int tdscha_check_errors(tdscha_ensemble *ens, void *stream);
  * (R1 (nb, n), Ys (nb, n, n) symmetric, device) and cotangents fbar (nb, n), Dbar (nb, n, n)
  * symmetric (device) it writes, summed over the nb vectors,
  *   Ybar (N, n)  = d[ sum_k <fbar_k, f_k> + <Dbar_k, D_k>_F ] / dY,   rhobar (N) = the same / drho
- * (device buffers, overwritten).  FP64 throughout; N_eff = sum(rho) is differentiated too.
+ * (device buffers, overwritten).  FP64 throughout; N_eff = sum(rho) is differentiated too.  At most
+ * 13760 modes (TDSCHA_EINVAL beyond).
  */
 int tdscha_perturb_average_vjp_device(tdscha_ensemble *ens, int nb, const double *R1, const double *Ys, int apply_d4,
                                       const double *fbar, const double *Dbar, double *Ybar, double *rhobar,

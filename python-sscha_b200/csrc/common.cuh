@@ -91,7 +91,8 @@ __device__ __forceinline__ float tf32_round(float f) {
 
 // Correctly rounded x / d from the rounded reciprocal of d: a product, its exact remainder and a
 // correction (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990,
-// theorem on quotients from a correctly rounded reciprocal); three FP64 instructions instead of a division.
+// theorem on quotients from a correctly rounded reciprocal); three FP64 instructions instead of a division.  Two differences
+// from a division, which no sum of such terms shows: -0 gives +0, and a quotient below the normal range may be a step off.
 __device__ __forceinline__ double div_by(double x, double d, double r) {   // r = 1 / d, correctly rounded
     const double q = x * r;
     const double c = __fma_rn(__fma_rn(-d, q, x), r, q);
